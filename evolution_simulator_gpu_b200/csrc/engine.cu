@@ -188,6 +188,18 @@ std::vector<unsigned> class_grids(ce_engine* e, const std::vector<ClassPlan>& pl
     return grids;
 }
 
+// Whether `count` creatures run on teams of lanes (team.cuh) instead of one
+// creature a lane. A launch of few creatures takes as long as its longest
+// trial, which teams shorten 2 to 7 times; a launch of many is bound by
+// instruction issue, of which a team spends about 2.4 times a lane's. The two
+// meet between 16,000 creatures of 3 to 6 nodes and 200,000 of 3 to 24 nodes
+// in the effects world (5 s trials, ms on teams / on lanes: small 16,384
+// 27.7 / 31.0 and 32,768 43.8 / 41.5; game 32,768 71 / 92 and 65,536 130 /
+// 108; effects 131,072 149 / 211 and 262,144 283 / 233). A caller that sets
+// the blocks an SM asks for the lane kernel's launch shape and gets it.
+constexpr size_t kTeamMost = 24576;
+bool team_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamMost; }
+
 ce_status check_world(const ce_world* w) {
     if (!w) {
         set_error("null world");
@@ -444,10 +456,11 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
     ce_make_params(w, 0, (uint32_t)pack->count, 0, &p);
     // Grids and scratch of the classes, which run side by side, each with its
     // own part of the slot's scratch.
-    const std::vector<unsigned> grids = class_grids(e, plans, flags, rate);
+    const bool team = team_pays(e, pack->count);
+    const std::vector<unsigned> grids = team ? std::vector<unsigned>(plans.size()) : class_grids(e, plans, flags, rate);
     std::vector<size_t> scratch_at(plans.size());
     size_t scratch = 0;
-    for (size_t c = 0; c < plans.size(); c++) {
+    for (size_t c = 0; c < plans.size() && !team; c++) {
         scratch_at[c] = scratch;
         scratch += (scratch_bytes(grids[c], plans[c].rows, plans[c].mm, false) + 255u) & ~(size_t)255u;
     }
@@ -471,6 +484,18 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
            "bucketing launch");
     CE_TRY(cudaEventRecord(sl.bucketed, st), "cudaEventRecord");
     CE_TRY(cudaStreamWaitEvent(sl.side, sl.bucketed, 0), "cudaStreamWaitEvent");
+    if (team) {
+        // One launch serves every node count.
+        ClassPlan all = plans.empty() ? ClassPlan{} : plans[0];
+        for (const ClassPlan& c : plans) {
+            all.last_n = std::max(all.last_n, c.last_n);
+            all.rows = std::max(all.rows, c.rows);
+            all.mm = std::max(all.mm, c.mm);
+        }
+        if (!plans.empty()) all.count = (uint32_t)pack->count;
+        plans.resize(std::min<size_t>(plans.size(), 1), all);
+        if (!plans.empty()) plans[0] = all;
+    }
     for (size_t c = 0; c < plans.size(); c++) {
         cek::KernelArgs a{};
         a.records = static_cast<const uint32_t*>(sl.d_lanes.ptr);
@@ -478,6 +503,7 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
         a.heads = static_cast<const uint4*>(sl.d_heads.ptr);
         a.results = static_cast<ce_result*>(sl.d_results.ptr);
         a.counter = bk.counters + plans[c].first_n;
+        a.first_n = plans[c].first_n;
         a.scratch = reinterpret_cast<float4*>(static_cast<char*>(sl.d_scratch.ptr) + scratch_at[c]);
         a.frames = nullptr;
         a.order = bk.order;
@@ -489,6 +515,11 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
         a.mm = plans[c].mm;
         a.frames_per_creature = 0;
         a.chunk_k = e->chunk_k;
+        if (team) {
+            const cek::TeamSpec ts{flags, rate, cek::team_blocks(a.rows, a.count), (unsigned)e->sms, st};
+            CE_TRY(cek::launch_team(ts, a, p), "advance launch");
+            continue;
+        }
         cek::LaunchSpec ls{plans[c].rows, plans[c].mm, flags, false, rate, grids[c], cek::kBlock,
                            c == 0 ? st : sl.side};
         CE_TRY(cek::launch_advance(ls, a, p), "advance launch");
@@ -627,8 +658,13 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
     a.mm = mm;
     a.frames_per_creature = per;
     a.chunk_k = 1;
-    cek::LaunchSpec ls{rows, mm, flags, true, rate, grid, cek::kBlock, nullptr};
-    CE_TRY(cek::launch_advance(ls, a, p), "record launch");
+    if (team_pays(e, pack->count)) {
+        const cek::TeamSpec ts{flags, rate, cek::team_blocks(rows, a.count), (unsigned)e->sms, nullptr};
+        CE_TRY(cek::launch_team_record(ts, a, p), "record launch");
+    } else {
+        cek::LaunchSpec ls{rows, mm, flags, true, rate, grid, cek::kBlock, nullptr};
+        CE_TRY(cek::launch_advance(ls, a, p), "record launch");
+    }
     CE_TRY(cek::launch_frames_to_creature_major(static_cast<const float2*>(e->rec_staging.ptr),
                                                 static_cast<float2*>(e->rec_frames.ptr), (size_t)per * stride,
                                                 (uint32_t)pack->count, nullptr),
@@ -700,6 +736,11 @@ ce_status advance_device(ce_engine* e, const uint32_t* records, const float* mus
         a.metrics = metrics;
         a.cells = cells;
         a.niche = *niche;
+    }
+    if (team_pays(e, params->count)) {
+        const cek::TeamSpec ts{world_flags, (int)rate, cek::team_blocks(max_nodes, a.count), (unsigned)e->sms, st};
+        CE_TRY(cek::launch_team(ts, a, *params), "advance launch");
+        return CE_OK;
     }
     cek::LaunchSpec ls{max_nodes, max_muscles, world_flags, false, (int)rate, grid, cek::kBlock, st};
     CE_TRY(cek::launch_advance(ls, a, *params), "advance launch");
@@ -872,7 +913,10 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     cek::KernelArgs a = tape_args(t, bk);
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
     cek::LaunchSpec ls{t->rows, t->mm, flags, false, t->rate, t->grid, cek::kBlock, st};
-    if ((s = cuda_status(cek::launch_forward_ckpt(ls, a, t->params), "forward launch")) ||
+    const cek::TeamSpec ts{flags, t->rate, cek::team_blocks(t->rows, a.count), (unsigned)e->sms, st};
+    if ((s = cuda_status(team_pays(e, a.count) ? cek::launch_team_ckpt(ts, a, t->params)
+                                               : cek::launch_forward_ckpt(ls, a, t->params),
+                         "forward launch")) ||
         (s = cuda_status(cudaEventRecord(t->stop, st), "cudaEventRecord")) ||
         (s = tape_time(t, &t->forward_seconds))) {
         return fail(s);
@@ -1277,7 +1321,9 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         const cek::LaunchSpec bs{a->rows, a->mm, flags, false, a->rate, bgrid, cek::kBlock, st};
         if (ce == cudaSuccess) ce = cek::launch_bucket(heads_d, 0u, (uint32_t)n, bk, st);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(a->d_ends.ptr, 0, n * 4, st);
-        if (ce == cudaSuccess) ce = cek::launch_forward_ckpt(fs, ka, a->params);
+        const cek::TeamSpec ts{flags, a->rate, cek::team_blocks(a->rows, n), (unsigned)e->sms, st};
+        if (ce == cudaSuccess)
+            ce = team_pays(e, n) ? cek::launch_team_ckpt(ts, ka, a->params) : cek::launch_forward_ckpt(fs, ka, a->params);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(a->d_grads.ptr, 0, n * per_grad * 4, st);
         if (ce == cudaSuccess) ce = cek::launch_bucket(heads_d, 0u, (uint32_t)n, bk, st);
         if (ce == cudaSuccess)
@@ -1307,7 +1353,8 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         ka.ckpt = nullptr;
         ka.ends = nullptr;
         const cek::LaunchSpec ls{a->rows, a->mm, flags, false, a->rate, fgrid, cek::kBlock, st};
-        ce = cek::launch_advance(ls, ka, a->params);
+        const cek::TeamSpec ts{flags, a->rate, cek::team_blocks(a->rows, n), (unsigned)e->sms, st};
+        ce = team_pays(e, n) ? cek::launch_team(ts, ka, a->params) : cek::launch_advance(ls, ka, a->params);
     }
     cudaGraph_t graph = nullptr;
     const ce_status end = cuda_status(cudaStreamEndCapture(st, &graph), "cudaStreamEndCapture");

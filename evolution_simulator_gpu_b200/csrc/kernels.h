@@ -52,6 +52,7 @@ struct KernelArgs {
     const uint32_t* order;         // packed positions of this launch's creatures
     const uint32_t* bounds;        // queues + 1 positions of the order list
     const unsigned long long* work;  // queues + 1 prefix sums of estimated work
+    uint32_t first_n;              // node count of queue 0
     uint32_t queues;               // 0: one queue, positions 0 .. count - 1
     uint32_t count;                // creatures of this launch
     uint32_t rows;                 // node rows: most nodes of a body of this launch
@@ -139,6 +140,22 @@ struct LaunchSpec {
     unsigned grid, block;
     cudaStream_t stream;
 };
+
+// Launches of the team kernels (team.cuh): plain trials, recordings and
+// checkpointed forward runs, on at most `blocks` blocks of kTeamBlock threads
+// (as many as fit the GPU's `sms` multiprocessors run).
+constexpr unsigned kTeamBlock = 64;
+constexpr unsigned kTeamMinBlocks = 8;
+struct TeamSpec {
+    uint32_t flags;
+    int rate;
+    unsigned blocks, sms;
+    cudaStream_t stream;
+};
+unsigned team_blocks(unsigned rows, size_t count);
+cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
+cudaError_t launch_team_record(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
+cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 
 // 16-byte lines of one lane's slot.
 unsigned slot_lines(unsigned rows, unsigned mm, bool record);

@@ -69,9 +69,11 @@ struct Clock {
 // time (RuntimeWorld). `has` of a compile-time world folds to a constant.
 template <uint32_t F>
 struct StaticWorld {
+    static constexpr bool fixed = true;
     __device__ __forceinline__ static constexpr bool has(uint32_t bit) { return (F & bit) != 0u; }
 };
 struct RuntimeWorld {
+    static constexpr bool fixed = false;
     uint32_t f;
     __device__ __forceinline__ bool has(uint32_t bit) const { return (f & bit) != 0u; }
 };

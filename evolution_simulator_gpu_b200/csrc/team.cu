@@ -1,0 +1,19 @@
+// Plain trials on teams of lanes (team.cuh).
+#include "team_launch.cuh"
+
+namespace cek {
+
+cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params& p) {
+    return s.rate == 60 ? team_in_world<false, 60>(s, a, p)
+           : s.rate == 120 ? team_in_world<false, 120>(s, a, p)
+                           : cudaErrorInvalidValue;
+}
+
+// Blocks of a launch that would give every creature its team at once.
+unsigned team_blocks(unsigned rows, size_t count) {
+    // Each team size may leave one warp partly filled.
+    const size_t blocks = (count * team_lanes(rows) + 3u * 32u + kTeamBlock - 1u) / kTeamBlock;
+    return (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
+}
+
+}  // namespace cek

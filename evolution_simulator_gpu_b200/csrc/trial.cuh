@@ -12,6 +12,303 @@ namespace cek {
 constexpr unsigned kFull = 0xffffffffu;
 static_assert(NodeTables::stride == kBlock, "node table rows are one block wide");
 
+// Centre of mass x, centre height, lowest and highest point and the
+// contact and lift bits of a step's end (shaders/creature.cu:1000-1023).
+struct Tally {
+    bool failed;
+    float center_y, com_x, low, high;
+    unsigned touching, lifted;
+};
+
+// The trial's metrics row and niche cell, from its 19 result words
+// (niche.cuh: the host's to_metrics and cell index to the bit).
+__device__ __forceinline__ void niche_epilogue(const KernelArgs& a, const LaneRegs& r, const float* m) {
+    const ce_result res{m[0],  m[1],  m[2],  m[3],  m[4],  m[5],  m[6],  m[7],  m[8], m[9],
+                        m[10], m[11], m[12], m[13], m[14], m[15], m[16], m[17], m[18]};
+    const ce_metrics mt = to_metrics(res, r.nodes, a.niche);
+    if (a.metrics) {
+        a.metrics[r.cidx] = mt;
+    }
+    a.cells[r.cidx] = cell_of(mt, r.nodes, a.shapes[r.cidx], a.niche);
+}
+
+// The lane words (the result and the tallies) at a trial's start: 0 except
+// the lowest and highest mean height and the head's position.
+__device__ __forceinline__ void start_words(float* lw, const float2& head) {
+#pragma unroll
+    for (unsigned q = 0u; q < 36u; q++) {
+        lw[q] = 0.0f;
+    }
+    lw[2] = 1e20f;
+    lw[3] = -1e20f;
+    lw[kWHeadAt] = head.x;
+    lw[kWHeadAt + 1u] = head.y;
+}
+
+// The end of a step: the tallies, the fall, the rungs, the screen and the
+// trial's end (shaders/creature.cu:1024-1248), from the step's `y` and
+// whether a joint is `broken`. `env` holds the creature's lane words, node
+// positions and energy stores. Returns whether the trial is over (a
+// recording goes on, limp).
+template <bool RECORD, bool CKPT, int RATE, class Env>
+__device__ __forceinline__ bool score(const Env& env, LaneRegs& r, const KernelArgs& a, const ce_params& p,
+                                      const Tally& y, bool broken) {
+    using C = Clock<RATE>;
+    const unsigned step = r.step;
+    const unsigned flags = r.flags;
+    const unsigned rung1 = (unsigned)(C::rate) - 1u, rung2 = (unsigned)(2.5f * C::rate) - 1u;
+    const unsigned rung3 = (unsigned)(5.0f * C::rate) - 1u, rung4 = (unsigned)(10.0f * C::rate) - 1u;
+    const unsigned half_s = (unsigned)(0.5f * C::rate);
+    const float t_now = __fmul_rn((float)step, C::dt);
+    const bool failed = y.failed;
+    float center_y = y.center_y, com_x = y.com_x;
+    const float low = y.low, high = y.high;
+    const unsigned touching = y.touching, lifted = y.lifted;
+    center_y /= (float)r.nodes;
+    com_x *= r.inv_mass;
+    // The result and tallies, from the lane lines.
+    // Words 0-18 are the result, 19-31 the tallies.
+    float lw[32];
+    env.load(lw);
+    float* const m = lw;
+    auto LW = [&](unsigned q) -> float& { return lw[q]; };
+    unsigned contact_bits = __float_as_uint(LW(kWContact));
+    unsigned lift_bits = __float_as_uint(LW(kWLift));
+    unsigned ground_bits = __float_as_uint(LW(kWGround));
+    float head_shake = LW(kWHeadShake);
+    float2 head_at = make_float2(LW(kWHeadAt), LW(kWHeadAt + 1u));
+    float2 head_vel = make_float2(LW(kWHeadVel), LW(kWHeadVel + 1u));
+    unsigned rung_x = __float_as_uint(LW(kWRungX));
+    unsigned rung_speed = __float_as_uint(LW(kWRungSpeed));
+    unsigned rung_early = __float_as_uint(LW(kWRungEarly));
+    unsigned rung_late = __float_as_uint(LW(kWRungLate));
+    unsigned rung_bits = __float_as_uint(LW(kWRungBits));
+    float& fitness = m[0];
+    float& ground_contact = m[1];
+    float& vertical_oscillation = m[2];
+    float& gait_frequency = m[3];
+    float& previous_center_y = m[4];
+    float& vertical_extremum = m[5];
+    float& vertical_trend = m[6];
+    float& gait_turns = m[7];
+    float& height_sum = m[8];
+    float& contact_lo = m[9];
+    float& contact_hi = m[10];
+    float& lift_lo = m[11];
+    float& lift_hi = m[12];
+    float& ground_lo = m[13];
+    float& ground_hi = m[14];
+    float& fall_time = m[15];
+    float& head_shake_r = m[16];
+    float& screen_x = m[17];
+    float& screened = m[18];
+
+    contact_bits |= touching;
+    lift_bits |= contact_bits & lifted;
+    const unsigned down = touching & ~ground_bits;
+    ground_bits = touching;
+    if (down != 0u && step > 0u) {
+        const float next = t_now + C::dt;
+        env.touchdown(down, next);
+    }
+    if ((step + 1u) % C::head_sample == 0u) {
+        const float2 h = env.pos(0u);
+        const float2 v = make_float2((h.x - head_at.x) * 60.0f, (h.y - head_at.y) * 60.0f);
+        const float ax = (v.x - head_vel.x) * 60.0f, ay = (v.y - head_vel.y) * 60.0f;
+        if (t_now >= kHeadShakeWindow) {
+            const float accel = sqrtf(ax * ax + ay * ay);
+            head_shake += (accel - head_shake) * fminf(1.0f / (kHeadShakeWindow * 60.0f), 1.0f);
+        }
+        head_at = h;
+        head_vel = v;
+    }
+    bool done = false;
+    if (!RECORD || r.scoring) {
+        contact_lo = __uint_as_float(contact_bits);
+        lift_lo = __uint_as_float(lift_bits);
+        ground_lo = __uint_as_float(ground_bits);
+        head_shake_r = head_shake;
+        const bool fell = env.pos(0u).y < env.pos(1u).y || broken || head_shake > kHeadShakeLimit || failed;
+        bool ended = false;
+        if (fell) {
+            fall_time = t_now + C::dt;
+            fitness = failed ? -1e20f : com_x;
+            if (step <= p.screen_step) {
+                screen_x = fitness;
+            }
+            ended = true;
+        }
+        ground_contact += (float)__popc(touching);
+        height_sum += high - low;
+        vertical_oscillation = fminf(vertical_oscillation, center_y);
+        gait_frequency = fmaxf(gait_frequency, center_y);
+        if (step == 0u) {
+            previous_center_y = center_y;
+            vertical_extremum = center_y;
+            vertical_trend = 0.0f;
+            gait_turns = 0.0f;
+        } else if (step % C::sample == 0u) {
+            const float delta = center_y - previous_center_y;
+            if (vertical_trend == 0.0f) {
+                if (fabsf(delta) > 0.0005f) {
+                    vertical_trend = delta > 0.0f ? 1.0f : -1.0f;
+                    vertical_extremum = center_y;
+                }
+            } else if (vertical_trend > 0.0f) {
+                if (center_y > vertical_extremum) {
+                    vertical_extremum = center_y;
+                } else if (vertical_extremum - center_y > 0.005f) {
+                    gait_turns += 1.0f;
+                    vertical_trend = -1.0f;
+                    vertical_extremum = center_y;
+                }
+            } else {
+                if (center_y < vertical_extremum) {
+                    vertical_extremum = center_y;
+                } else if (center_y - vertical_extremum > 0.005f) {
+                    gait_turns += 1.0f;
+                    vertical_trend = 1.0f;
+                    vertical_extremum = center_y;
+                }
+            }
+            previous_center_y = center_y;
+        }
+        if (step + half_s == rung1 || step + half_s == rung2) {
+            rung_x = __float_as_uint(com_x);
+        }
+        if (step == rung1 || step == rung2) {
+            const bool second = step == rung2;
+            const unsigned sh = second ? 16u : 0u;
+            const unsigned keep = second ? 0x0000ffffu : 0xffff0000u;
+            const float speed = (com_x - __uint_as_float(rung_x)) * (C::rate / (float)half_s);
+            const float touched = (float)__popc(contact_bits) / (float)r.nodes;
+            float en_mean = 0.0f;
+            for (unsigned k = 0u; k < r.muscles; k++) {
+                en_mean += env.energy(k);
+            }
+            en_mean /= (float)max(r.muscles, 1u);
+            contact_hi = __uint_as_float((__float_as_uint(contact_hi) & keep) | (f2h(com_x) << sh));
+            ground_hi = __uint_as_float((__float_as_uint(ground_hi) & keep) | (f2h(head_shake) << sh));
+            rung_speed = (rung_speed & keep) | (f2h(speed) << sh);
+            const unsigned pair = f2h(touched) | (f2h(en_mean) << 16u);
+            if (second) {
+                rung_late = pair;
+            } else {
+                rung_early = pair;
+            }
+            const unsigned rr = second ? 1u : 0u;
+            const float gait_now = gait_turns * (0.5f / (t_now + C::dt));
+            const unsigned band = min((unsigned)(gait_now * (8.0f / 6.0f)), 7u);
+            rung_bits |= band << (8u + 3u * rr);
+            if (!ended && (flags & (second ? 0xbu : 0x7u)) == 0u) {
+                const ce_rung& rp = second ? p.r2 : p.r1;
+                const float fv[6] = {h2f(f2h(com_x)),      h2f(f2h(speed)),   h2f(f2h(touched)),
+                                     h2f(f2h(head_shake)), h2f(f2h(en_mean)), r.period_f};
+                float score = 0.0f;
+                bool finite = true;
+                for (int i = 0; i < 6; i++) {
+                    score = fmaf(rp.w[i], fv[i], score);
+                    finite = finite && isfinite(fv[i]);
+                }
+                if (finite && score < rp.bias && ((rp.off >> band) & 1u) == 0u) {
+                    screened = t_now + C::dt;
+                    screen_x = com_x;
+                    fitness = com_x;
+                    rung_bits |= (rr + 1u) << 6u;
+                    ended = true;
+                }
+            }
+        }
+        if (step == rung3 || step == rung4) {
+            const bool second = step == rung4;
+            const unsigned keep = second ? 0x0000ffffu : 0xffff0000u;
+            lift_hi = __uint_as_float((__float_as_uint(lift_hi) & keep) | (f2h(com_x) << (second ? 16u : 0u)));
+        }
+        if (step == p.screen_step && !ended) {
+            screen_x = com_x;
+            const float bar = (flags & 32u) != 0u   ? p.screen_bar_reshaped
+                              : (flags & 16u) != 0u ? p.screen_bar_young
+                                                    : p.screen_bar;
+            if (com_x < bar && (flags & 1u) == 0u) {
+                screened = t_now + C::dt;
+                fitness = com_x;
+                ended = true;
+            }
+        }
+        bool last = false;
+        if (ended) {
+            vertical_oscillation = fmaxf(gait_frequency - vertical_oscillation, 0.0f);
+            gait_frequency = gait_turns * 0.5f / (t_now + C::dt);
+        } else if (step + 1u >= p.steps) {
+            fitness = com_x;
+            vertical_oscillation = fmaxf(gait_frequency - vertical_oscillation, 0.0f);
+            gait_frequency = gait_turns * 0.5f / fmaxf((float)(step + 1u) * C::dt, C::dt);
+            last = true;
+        }
+        if (ended || last) {
+            const unsigned fin = f2h(fitness);
+            unsigned d = __float_as_uint(contact_hi);
+            if (step < rung1) {
+                d = (d & 0xffff0000u) | fin;
+            }
+            if (step < rung2) {
+                d = (d & 0x0000ffffu) | (fin << 16u);
+            }
+            contact_hi = __uint_as_float(d);
+            d = __float_as_uint(lift_hi);
+            if (step < rung3) {
+                d = (d & 0xffff0000u) | fin;
+            }
+            if (step < rung4) {
+                d = (d & 0x0000ffffu) | (fin << 16u);
+            }
+            lift_hi = __uint_as_float(d);
+            const unsigned code = (fell ? 16u : 0u) | (failed ? 32u : 0u) | (screened > 0.0f ? 3u : 0u) |
+                                  (rung_bits & 0x3fc0u) | ((flags & 1u) << 14u);
+            previous_center_y = __uint_as_float(rung_speed);
+            vertical_extremum = __uint_as_float(rung_early);
+            vertical_trend = __uint_as_float(rung_late);
+            gait_turns = ground_hi;
+            ground_hi = __uint_as_float(code | (min(step + 1u, 65535u) << 16u));
+            if (RECORD) {
+                env.keep(m);
+                r.scoring = false;
+                r.limp = true;
+            } else {
+                float* out = reinterpret_cast<float*>(a.results + r.cidx);
+                for (unsigned q = 0u; q < 19u; q++) {
+                    __stcs(out + q, m[q]);
+                }
+                if (!CKPT && a.cells) {
+                    niche_epilogue(a, r, m);
+                }
+                if (CKPT) {
+                    a.ends[r.cidx] = step + 1u;
+                }
+                done = true;
+            }
+        }
+    }
+    if (done) {
+        return true;
+    }
+    LW(kWContact) = __uint_as_float(contact_bits);
+    LW(kWLift) = __uint_as_float(lift_bits);
+    LW(kWGround) = __uint_as_float(ground_bits);
+    LW(kWHeadShake) = head_shake;
+    LW(kWHeadAt) = head_at.x;
+    LW(kWHeadAt + 1u) = head_at.y;
+    LW(kWHeadVel) = head_vel.x;
+    LW(kWHeadVel + 1u) = head_vel.y;
+    LW(kWRungX) = __uint_as_float(rung_x);
+    LW(kWRungSpeed) = __uint_as_float(rung_speed);
+    LW(kWRungEarly) = __uint_as_float(rung_early);
+    LW(kWRungLate) = __uint_as_float(rung_late);
+    LW(kWRungBits) = __uint_as_float(rung_bits);
+    env.store(lw);
+    return false;
+}
+
 template <class W, bool RECORD, int RATE, bool CKPT = false>
 struct Trial {
     using C = Clock<RATE>;
@@ -147,17 +444,8 @@ struct Trial {
                 L.word(S.rec_pull + k / 4u, k % 4u) = 0.0f;
             }
         }
-        // The result starts at 0 except the lowest and highest mean height.
-        const float2 head = b.t.pos(0u);
         float lw[36];
-#pragma unroll
-        for (unsigned q = 0u; q < 36u; q++) {
-            lw[q] = 0.0f;
-        }
-        lw[2] = 1e20f;
-        lw[3] = -1e20f;
-        lw[kWHeadAt] = head.x;
-        lw[kWHeadAt + 1u] = head.y;
+        start_words(lw, b.t.pos(0u));
 #pragma unroll
         for (unsigned q = 0u; q < 9u; q++) {
             L.put_cold(S.lane + q, make_float4(lw[4u * q], lw[4u * q + 1u], lw[4u * q + 2u], lw[4u * q + 3u]));
@@ -172,13 +460,6 @@ struct Trial {
         }
     }
 
-    // Centre of mass x, centre height, lowest and highest point and the
-    // contact and lift bits of the step's end (shaders/creature.cu:1000-1023).
-    struct Tally {
-        bool failed;
-        float center_y, com_x, low, high;
-        unsigned touching, lifted;
-    };
     __device__ __forceinline__ static void tally_node(const Body& b, Tally& y, unsigned i, const float4& nr) {
         const float2 q = b.t.pos(i);
         y.failed = y.failed || !(fabsf(q.x) <= 1e6f && fabsf(q.y) <= 1e6f);
@@ -205,17 +486,44 @@ struct Trial {
         return y;
     }
 
-    // The trial's metrics row and niche cell, from its 19 result words
-    // (niche.cuh: the host's to_metrics and cell index to the bit).
-    __device__ __forceinline__ static void niche_epilogue(const KernelArgs& a, const LaneRegs& r, const float* m) {
-        const ce_result res{m[0],  m[1],  m[2],  m[3],  m[4],  m[5],  m[6],  m[7],  m[8], m[9],
-                            m[10], m[11], m[12], m[13], m[14], m[15], m[16], m[17], m[18]};
-        const ce_metrics mt = to_metrics(res, r.nodes, a.niche);
-        if (a.metrics) {
-            a.metrics[r.cidx] = mt;
+    // Where this lane keeps what score() reads and writes.
+    struct Words {
+        const Body& b;
+        __device__ __forceinline__ float2 pos(unsigned i) const { return b.t.pos(i); }
+        __device__ __forceinline__ float energy(unsigned k) const { return b.t.muscle(k).x; }
+        __device__ __forceinline__ void load(float* lw) const {
+#pragma unroll
+            for (unsigned q = 0u; q < 8u; q++) {
+                const float4 v = b.L.get_cold(b.S.lane + q);
+                lw[4u * q] = v.x;
+                lw[4u * q + 1u] = v.y;
+                lw[4u * q + 2u] = v.z;
+                lw[4u * q + 3u] = v.w;
+            }
         }
-        a.cells[r.cidx] = cell_of(mt, r.nodes, a.shapes[r.cidx], a.niche);
-    }
+        __device__ __forceinline__ void store(const float* lw) const {
+#pragma unroll
+            for (unsigned q = 0u; q < 8u; q++) {
+                b.L.put_cold(b.S.lane + q, make_float4(lw[4u * q], lw[4u * q + 1u], lw[4u * q + 2u], lw[4u * q + 3u]));
+            }
+        }
+        // A touch sensor among the nodes `down` restarts its muscle's rhythm.
+        __device__ __forceinline__ void touchdown(unsigned down, float next) const {
+            for (unsigned k = 0u; k < b.r.muscles; k++) {
+                const unsigned m0 = b.S.muscle + 5u * k;
+                const unsigned sensor = __float_as_uint(b.L.word_cold(m0 + kMState, 3));
+                if (sensor != kNone && ((down >> sensor) & 1u)) {
+                    const float4 r0 = b.L.get_cold(m0 + kRhythm0), r1 = b.L.get_cold(m0 + kRhythm1);
+                    b.L.set_cold(m0 + kMState, 2, fracf(r1.w - (next * r0.y + r0.z)));
+                }
+            }
+        }
+        __device__ __forceinline__ void keep(const float* m) const {
+            for (unsigned q = 0u; q < 19u; q++) {
+                b.L.word(b.S.rec_kept + q / 4u, q % 4u) = m[q];
+            }
+        }
+    };
 
     // One step of the creature on this lane (shaders/creature.cu:956-1248).
     // Returns whether the lane still has a creature.
@@ -225,10 +533,6 @@ struct Trial {
         const Lines& L = b.L;
         const SlotLayout& S = b.S;
         const unsigned step = r.step;
-        const unsigned flags = r.flags;
-        const unsigned rung1 = (unsigned)(C::rate) - 1u, rung2 = (unsigned)(2.5f * C::rate) - 1u;
-        const unsigned rung3 = (unsigned)(5.0f * C::rate) - 1u, rung4 = (unsigned)(10.0f * C::rate) - 1u;
-        const unsigned half_s = (unsigned)(0.5f * C::rate);
         const float t_now = (float)step * C::dt;
         if (RECORD) {
             for (unsigned i = 0u; i < r.nodes; i++) {
@@ -252,270 +556,8 @@ struct Trial {
         }
         const Tally y = tally(b);
         const bool broken = b.broken_joints() != 0ull;
-        const bool failed = y.failed;
-        float center_y = y.center_y, com_x = y.com_x;
-        const float low = y.low, high = y.high;
-        const unsigned touching = y.touching, lifted = y.lifted;
-        center_y /= (float)r.nodes;
-        com_x *= r.inv_mass;
-        // The result and tallies, from the lane lines.
-        // Words 0-18 are the result, 19-31 the tallies.
-        float lw[32];
-#pragma unroll
-        for (unsigned q = 0u; q < 8u; q++) {
-            const float4 v = L.get_cold(S.lane + q);
-            lw[4u * q] = v.x;
-            lw[4u * q + 1u] = v.y;
-            lw[4u * q + 2u] = v.z;
-            lw[4u * q + 3u] = v.w;
-        }
-        float* const m = lw;
-        auto LW = [&](unsigned q) -> float& { return lw[q]; };
-        unsigned contact_bits = __float_as_uint(LW(kWContact));
-        unsigned lift_bits = __float_as_uint(LW(kWLift));
-        unsigned ground_bits = __float_as_uint(LW(kWGround));
-        float head_shake = LW(kWHeadShake);
-        float2 head_at = make_float2(LW(kWHeadAt), LW(kWHeadAt + 1u));
-        float2 head_vel = make_float2(LW(kWHeadVel), LW(kWHeadVel + 1u));
-        unsigned rung_x = __float_as_uint(LW(kWRungX));
-        unsigned rung_speed = __float_as_uint(LW(kWRungSpeed));
-        unsigned rung_early = __float_as_uint(LW(kWRungEarly));
-        unsigned rung_late = __float_as_uint(LW(kWRungLate));
-        unsigned rung_bits = __float_as_uint(LW(kWRungBits));
-        float& fitness = m[0];
-        float& ground_contact = m[1];
-        float& vertical_oscillation = m[2];
-        float& gait_frequency = m[3];
-        float& previous_center_y = m[4];
-        float& vertical_extremum = m[5];
-        float& vertical_trend = m[6];
-        float& gait_turns = m[7];
-        float& height_sum = m[8];
-        float& contact_lo = m[9];
-        float& contact_hi = m[10];
-        float& lift_lo = m[11];
-        float& lift_hi = m[12];
-        float& ground_lo = m[13];
-        float& ground_hi = m[14];
-        float& fall_time = m[15];
-        float& head_shake_r = m[16];
-        float& screen_x = m[17];
-        float& screened = m[18];
-
-        contact_bits |= touching;
-        lift_bits |= contact_bits & lifted;
-        const unsigned down = touching & ~ground_bits;
-        ground_bits = touching;
-        if (down != 0u && step > 0u) {
-            const float next = t_now + C::dt;
-            for (unsigned k = 0u; k < r.muscles; k++) {
-                const unsigned m0 = S.muscle + 5u * k;
-                const unsigned sensor = __float_as_uint(L.word_cold(m0 + kMState, 3));
-                if (sensor != kNone && ((down >> sensor) & 1u)) {
-                    const float4 r0 = L.get_cold(m0 + kRhythm0), r1 = L.get_cold(m0 + kRhythm1);
-                    L.set_cold(m0 + kMState, 2, fracf(r1.w - (next * r0.y + r0.z)));
-                }
-            }
-        }
-        if ((step + 1u) % C::head_sample == 0u) {
-            const float2 h = b.t.pos(0u);
-            const float2 v = make_float2((h.x - head_at.x) * 60.0f, (h.y - head_at.y) * 60.0f);
-            const float ax = (v.x - head_vel.x) * 60.0f, ay = (v.y - head_vel.y) * 60.0f;
-            if (t_now >= kHeadShakeWindow) {
-                const float accel = sqrtf(ax * ax + ay * ay);
-                head_shake += (accel - head_shake) * fminf(1.0f / (kHeadShakeWindow * 60.0f), 1.0f);
-            }
-            head_at = h;
-            head_vel = v;
-        }
-        bool done = false;
-        if (!RECORD || r.scoring) {
-            contact_lo = __uint_as_float(contact_bits);
-            lift_lo = __uint_as_float(lift_bits);
-            ground_lo = __uint_as_float(ground_bits);
-            head_shake_r = head_shake;
-            const bool fell = b.t.pos(0u).y < b.t.pos(1u).y || broken || head_shake > kHeadShakeLimit || failed;
-            bool ended = false;
-            if (fell) {
-                fall_time = t_now + C::dt;
-                fitness = failed ? -1e20f : com_x;
-                if (step <= p.screen_step) {
-                    screen_x = fitness;
-                }
-                ended = true;
-            }
-            ground_contact += (float)__popc(touching);
-            height_sum += high - low;
-            vertical_oscillation = fminf(vertical_oscillation, center_y);
-            gait_frequency = fmaxf(gait_frequency, center_y);
-            if (step == 0u) {
-                previous_center_y = center_y;
-                vertical_extremum = center_y;
-                vertical_trend = 0.0f;
-                gait_turns = 0.0f;
-            } else if (step % C::sample == 0u) {
-                const float delta = center_y - previous_center_y;
-                if (vertical_trend == 0.0f) {
-                    if (fabsf(delta) > 0.0005f) {
-                        vertical_trend = delta > 0.0f ? 1.0f : -1.0f;
-                        vertical_extremum = center_y;
-                    }
-                } else if (vertical_trend > 0.0f) {
-                    if (center_y > vertical_extremum) {
-                        vertical_extremum = center_y;
-                    } else if (vertical_extremum - center_y > 0.005f) {
-                        gait_turns += 1.0f;
-                        vertical_trend = -1.0f;
-                        vertical_extremum = center_y;
-                    }
-                } else {
-                    if (center_y < vertical_extremum) {
-                        vertical_extremum = center_y;
-                    } else if (center_y - vertical_extremum > 0.005f) {
-                        gait_turns += 1.0f;
-                        vertical_trend = 1.0f;
-                        vertical_extremum = center_y;
-                    }
-                }
-                previous_center_y = center_y;
-            }
-            if (step + half_s == rung1 || step + half_s == rung2) {
-                rung_x = __float_as_uint(com_x);
-            }
-            if (step == rung1 || step == rung2) {
-                const bool second = step == rung2;
-                const unsigned sh = second ? 16u : 0u;
-                const unsigned keep = second ? 0x0000ffffu : 0xffff0000u;
-                const float speed = (com_x - __uint_as_float(rung_x)) * (C::rate / (float)half_s);
-                const float touched = (float)__popc(contact_bits) / (float)r.nodes;
-                float en_mean = 0.0f;
-                for (unsigned k = 0u; k < r.muscles; k++) {
-                    en_mean += b.t.muscle(k).x;
-                }
-                en_mean /= (float)max(r.muscles, 1u);
-                contact_hi = __uint_as_float((__float_as_uint(contact_hi) & keep) | (f2h(com_x) << sh));
-                ground_hi = __uint_as_float((__float_as_uint(ground_hi) & keep) | (f2h(head_shake) << sh));
-                rung_speed = (rung_speed & keep) | (f2h(speed) << sh);
-                const unsigned pair = f2h(touched) | (f2h(en_mean) << 16u);
-                if (second) {
-                    rung_late = pair;
-                } else {
-                    rung_early = pair;
-                }
-                const unsigned rr = second ? 1u : 0u;
-                const float gait_now = gait_turns * (0.5f / (t_now + C::dt));
-                const unsigned band = min((unsigned)(gait_now * (8.0f / 6.0f)), 7u);
-                rung_bits |= band << (8u + 3u * rr);
-                if (!ended && (flags & (second ? 0xbu : 0x7u)) == 0u) {
-                    const ce_rung& rp = second ? p.r2 : p.r1;
-                    const float fv[6] = {h2f(f2h(com_x)),      h2f(f2h(speed)),   h2f(f2h(touched)),
-                                         h2f(f2h(head_shake)), h2f(f2h(en_mean)), r.period_f};
-                    float score = 0.0f;
-                    bool finite = true;
-                    for (int i = 0; i < 6; i++) {
-                        score = fmaf(rp.w[i], fv[i], score);
-                        finite = finite && isfinite(fv[i]);
-                    }
-                    if (finite && score < rp.bias && ((rp.off >> band) & 1u) == 0u) {
-                        screened = t_now + C::dt;
-                        screen_x = com_x;
-                        fitness = com_x;
-                        rung_bits |= (rr + 1u) << 6u;
-                        ended = true;
-                    }
-                }
-            }
-            if (step == rung3 || step == rung4) {
-                const bool second = step == rung4;
-                const unsigned keep = second ? 0x0000ffffu : 0xffff0000u;
-                lift_hi = __uint_as_float((__float_as_uint(lift_hi) & keep) | (f2h(com_x) << (second ? 16u : 0u)));
-            }
-            if (step == p.screen_step && !ended) {
-                screen_x = com_x;
-                const float bar = (flags & 32u) != 0u   ? p.screen_bar_reshaped
-                                  : (flags & 16u) != 0u ? p.screen_bar_young
-                                                        : p.screen_bar;
-                if (com_x < bar && (flags & 1u) == 0u) {
-                    screened = t_now + C::dt;
-                    fitness = com_x;
-                    ended = true;
-                }
-            }
-            bool last = false;
-            if (ended) {
-                vertical_oscillation = fmaxf(gait_frequency - vertical_oscillation, 0.0f);
-                gait_frequency = gait_turns * 0.5f / (t_now + C::dt);
-            } else if (step + 1u >= p.steps) {
-                fitness = com_x;
-                vertical_oscillation = fmaxf(gait_frequency - vertical_oscillation, 0.0f);
-                gait_frequency = gait_turns * 0.5f / fmaxf((float)(step + 1u) * C::dt, C::dt);
-                last = true;
-            }
-            if (ended || last) {
-                const unsigned fin = f2h(fitness);
-                unsigned d = __float_as_uint(contact_hi);
-                if (step < rung1) {
-                    d = (d & 0xffff0000u) | fin;
-                }
-                if (step < rung2) {
-                    d = (d & 0x0000ffffu) | (fin << 16u);
-                }
-                contact_hi = __uint_as_float(d);
-                d = __float_as_uint(lift_hi);
-                if (step < rung3) {
-                    d = (d & 0xffff0000u) | fin;
-                }
-                if (step < rung4) {
-                    d = (d & 0x0000ffffu) | (fin << 16u);
-                }
-                lift_hi = __uint_as_float(d);
-                const unsigned code = (fell ? 16u : 0u) | (failed ? 32u : 0u) | (screened > 0.0f ? 3u : 0u) |
-                                      (rung_bits & 0x3fc0u) | ((flags & 1u) << 14u);
-                previous_center_y = __uint_as_float(rung_speed);
-                vertical_extremum = __uint_as_float(rung_early);
-                vertical_trend = __uint_as_float(rung_late);
-                gait_turns = ground_hi;
-                ground_hi = __uint_as_float(code | (min(step + 1u, 65535u) << 16u));
-                if (RECORD) {
-                    for (unsigned q = 0u; q < 19u; q++) {
-                        L.word(S.rec_kept + q / 4u, q % 4u) = m[q];
-                    }
-                    r.scoring = false;
-                    r.limp = true;
-                } else {
-                    float* out = reinterpret_cast<float*>(a.results + r.cidx);
-                    for (unsigned q = 0u; q < 19u; q++) {
-                        __stcs(out + q, m[q]);
-                    }
-                    if (!CKPT && a.cells) {
-                        niche_epilogue(a, r, m);
-                    }
-                    if (CKPT) {
-                        a.ends[r.cidx] = step + 1u;
-                    }
-                    done = true;
-                }
-            }
-        }
-        if (done) {
+        if (score<RECORD, CKPT, RATE>(Words{b}, r, a, p, y, broken)) {
             return false;
-        }
-        LW(kWContact) = __uint_as_float(contact_bits);
-        LW(kWLift) = __uint_as_float(lift_bits);
-        LW(kWGround) = __uint_as_float(ground_bits);
-        LW(kWHeadShake) = head_shake;
-        LW(kWHeadAt) = head_at.x;
-        LW(kWHeadAt + 1u) = head_at.y;
-        LW(kWHeadVel) = head_vel.x;
-        LW(kWHeadVel + 1u) = head_vel.y;
-        LW(kWRungX) = __uint_as_float(rung_x);
-        LW(kWRungSpeed) = __uint_as_float(rung_speed);
-        LW(kWRungEarly) = __uint_as_float(rung_early);
-        LW(kWRungLate) = __uint_as_float(rung_late);
-        LW(kWRungBits) = __uint_as_float(rung_bits);
-#pragma unroll
-        for (unsigned q = 0u; q < 8u; q++) {
-            L.put_cold(S.lane + q, make_float4(lw[4u * q], lw[4u * q + 1u], lw[4u * q + 2u], lw[4u * q + 3u]));
         }
         if (RECORD) {
             record_frame(b, a, C::settle + step + 1u);
