@@ -8,13 +8,12 @@
 // least power of two that gives every node a lane) runs one creature:
 //
 // * lane i holds node i, the bone that ends there and that bone's joint, with
-//   their constants and the node's position and velocity in registers;
+//   their constants in registers and its state in shared memory;
 // * the muscles go round the lanes; their forces meet in shared memory and
 //   each node's lane adds up its own in the muscles' order (a list built when
 //   the trial begins), so a sum has the serial pass's rounding;
 // * the bones' drag and lengths, which update two nodes each in bone order,
-//   run in levels: a bone goes when the last earlier bone at its pivot has,
-//   and takes the pivot's value from that bone's lane by a shuffle. Levels
+//   run in levels: a bone goes when every earlier bone at its nodes has. Levels
 //   are the depth of the body's left-child right-sibling tree (3 to 6 for 6
 //   to 10 nodes) instead of its bone count. The damping runs in levels too,
 //   over the joints that share a node;
@@ -194,16 +193,13 @@ struct Team {
 
     // Node i, bone i - 1 (pivot to node i), its joint.
     float4 nr, ba, bb, ra, rb;
-    float2 p, v;
     float2 shown_force;                  // RECORD: contact forces summed over a step
     unsigned e0 = 0u, e1 = 0u;           // the node's entries
-    unsigned prior = 0u, last = 0u;      // lanes that hold the pivot's value before this bone, the node's after all
-    bool prior_pivot = false, has_last = false;
     unsigned level = 0u, damp_level = 0u;  // 0: no bone, no joint
     unsigned before = 0u;                // lanes whose joints this one's test depends on
     unsigned levels = 0u, damp_levels = 0u;  // the warp's most
     unsigned rhythm_at = 0u;             // the creature's muscle records
-    bool in_order = true;                // a tree in every team: pivots before their bones' ends, joints of three nodes
+    bool distinct = true;                // every joint of the warp's bodies joins three nodes
 
     __device__ __forceinline__ float2& pos(unsigned n) const { return reinterpret_cast<float2*>(mem)[n]; }
     __device__ __forceinline__ float2& vel(unsigned n) const { return reinterpret_cast<float2*>(mem + S.vel)[n]; }
@@ -233,7 +229,7 @@ struct Team {
         mem = warp_mem + (base / T) * S.bytes;
         nr = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
         ba = bb = ra = rb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        p = v = shown_force = make_float2(0.0f, 0.0f);
+        shown_force = make_float2(0.0f, 0.0f);
         r = LaneRegs{};
         leave();
     }
@@ -244,9 +240,7 @@ struct Team {
         level = 0u;
         damp_level = 0u;
         e0 = e1 = 0u;
-        has_last = false;
         before = 0u;
-        prior = 0u;
         ra.x = __uint_as_float(kNone);
     }
 
@@ -290,16 +284,12 @@ struct Team {
                 const uint32_t* q = rec + i * CE_NODE_WORDS;
                 const float m = __uint_as_float(__ldcs(q + 0));
                 new_nr = make_float4(m, 1.0f / m, __uint_as_float(__ldcs(q + 1)), __uint_as_float(__ldcs(q + 2)));
-                p = make_float2(__uint_as_float(__ldcs(q + 3)), __uint_as_float(__ldcs(q + 4)));
+                pos(i) = make_float2(__uint_as_float(__ldcs(q + 3)), __uint_as_float(__ldcs(q + 4)));
+                vel(i) = make_float2(0.0f, 0.0f);
                 foot = (__ldcs(q + 5) & 1u) != 0u;
                 tally_of(i) = make_float2(new_nr.x, new_nr.z);
-            } else {
-                p = make_float2(0.0f, 0.0f);
             }
-            v = make_float2(0.0f, 0.0f);
             shown_force = make_float2(0.0f, 0.0f);
-            pos(i) = p;
-            vel(i) = v;
         }
         const unsigned feet = votes(foot);
         if (fresh) r.feet = feet;
@@ -358,7 +348,7 @@ struct Team {
             }
             if (i == 0u) {
                 float lw[36];
-                start_words(lw, p);
+                start_words(lw, pos(0u));
                 for (unsigned q = 0u; q < 32u; q++) {
                     words()[q] = lw[q];
                 }
@@ -390,31 +380,16 @@ struct Team {
                 }
             }
         }
-        // Levels: of the bones by the pivot's last earlier bone, of the
-        // joints by the nodes that they share.
+        // Levels: an item's is one past the largest of the earlier items that
+        // share a node with it.
         const bool bone = fresh && has_bone(), joint = fresh && writes != 0u;
         unsigned level_now = bone ? 1u : 0u, damp_now = joint ? 1u : 0u, anc = 0u;
-        unsigned prior_now = pivot, last_now = 0u;
-        bool prior_pivot_now = false, has_last_now = false;
-        for (unsigned s = 1u; s < T; s++) {
-            const unsigned ps = from(bone ? pivot : kNone, s);
-            if (ps == kNone) {
-                continue;
-            }
-            if (s < i && bone && ps == pivot) {
-                prior_now = s;
-                prior_pivot_now = true;
-            }
-            if (fresh && has_node() && ps == i) {
-                last_now = s;
-                has_last_now = true;
-            }
-        }
+        const unsigned ends = bone ? (1u << i) | (1u << pivot) : 0u;
         for (unsigned s = 1u; s < T; s++) {
             const unsigned ls = from(level_now, s), ds = from(damp_now, s), as = from(anc, s);
-            const unsigned ws = from(writes, s), rs = from(reads, s);
-            if (s < i && bone && prior_now == s) {
-                level_now = ls + 1u;
+            const unsigned es = from(ends, s), ws = from(writes, s), rs = from(reads, s);
+            if (s < i && (es & ends) != 0u) {
+                level_now = max(level_now, ls + 1u);
             }
             if (s < i && joint && ws != 0u) {
                 if (((ws & reads) | (rs & writes)) != 0u) {
@@ -429,17 +404,12 @@ struct Team {
             level = level_now;
             damp_level = damp_now;
             before = anc;
-            prior = prior_now;
-            prior_pivot = prior_pivot_now;
-            last = last_now;
-            has_last = has_last_now;
         }
         levels = __reduce_max_sync(kFull, level);
         damp_levels = __reduce_max_sync(kFull, damp_level);
         const unsigned topo = __float_as_uint(ra.x);
-        in_order = __all_sync(kFull, !has_bone() ||
-                                         (__float_as_uint(ba.x) < i &&
-                                          (!has_joint() || (((topo >> 15u) & 31u) != i && ((topo >> 15u) & 31u) != (topo & 31u)))));
+        distinct = __all_sync(kFull, !has_joint() || (((topo >> 15u) & 31u) != i &&
+                                                      ((topo >> 15u) & 31u) != (topo & 31u) && (topo & 31u) != i));
         __syncwarp();
         if (RECORD) {
             for (unsigned t = 0u; t <= C::settle; t++) {
@@ -476,7 +446,7 @@ struct Team {
         const size_t k = a.count;
         float2* fr = a.frames + (size_t)t * stride * k + r.rec_slot;
         if (has_node()) {
-            fr[i * k] = p;
+            fr[i * k] = pos(i);
             fr[(CE_MAX_NODES + r.muscles + i) * k] = shown_force;
         }
         for (unsigned m = i; m < r.muscles; m += T) {
@@ -493,6 +463,7 @@ struct Team {
         const size_t count = a.count;
         float* c = a.ckpt + (size_t)n * checkpoint_floats(a.rows, a.mm) * count + r.cidx;
         if (has_node()) {
+            const float2 p = pos(i), v = vel(i);
             __stcs(c + (2u * i) * count, p.x);
             __stcs(c + (2u * i + 1u) * count, p.y);
             __stcs(c + (2u * a.rows + 2u * i) * count, v.x);
@@ -504,20 +475,35 @@ struct Team {
     }
 
     __device__ __forceinline__ bool has_joint() const { return __float_as_uint(ra.x) != kNone; }
-    // The joint of this lane from the positions in shared memory.
-    template <bool LIMIT>
+    // The joint of this lane from the positions in shared memory, its angle,
+    // and how far that is past its range (0 within it).
     __device__ __forceinline__ Joint joint() const {
         const unsigned topo = __float_as_uint(ra.x);
-        return P::template joint_at<LIMIT>(i - 1u, ra, rb, pos((topo >> 5u) & 31u), pos((topo >> 10u) & 31u), pos(i),
-                                           pos(topo & 31u));
+        return P::joint_at(i - 1u, ra, rb, pos((topo >> 5u) & 31u), pos((topo >> 10u) & 31u), pos(i),
+                           pos(topo & 31u));
     }
-    template <bool VEL>
-    __device__ __forceinline__ void push(const Joint& k, float lambda) const {
-        float2& tip = VEL ? vel(k.tip) : pos(k.tip);
-        float2& far = VEL ? vel(k.far) : pos(k.far);
-        float2& hub = VEL ? vel(k.hub) : pos(k.hub);
+    __device__ __forceinline__ float angle() const {
+        const unsigned topo = __float_as_uint(ra.x);
+        return P::angle_at(ra, pos((topo >> 5u) & 31u), pos((topo >> 10u) & 31u), pos(i), pos(topo & 31u));
+    }
+    __device__ __forceinline__ float joint_error() const {
+        const float x = angle();
+        float error = 0.0f;
+        if (x < ra.y) {
+            error = x - ra.y;
+        }
+        if (x > ra.z) {
+            error = x - ra.z;
+        }
+        return error;
+    }
+    // Moves the joint's three nodes in `table` along its gradients.
+    __device__ __forceinline__ void push(const Joint& k, float lambda, float2* table) const {
+        float2& tip = table[k.tip];
+        float2& far = table[k.far];
+        float2& hub = table[k.hub];
         float2 e = tip;
-        if (!in_order) {
+        if (!distinct) {
             // Two of the three may be one node: one after the other.
             tip = make_float2(__fmaf_rn(__fmul_rn(k.w_tip, lambda), k.g_tip.x, e.x),
                               __fmaf_rn(__fmul_rn(k.w_tip, lambda), k.g_tip.y, e.y));
@@ -546,8 +532,8 @@ struct Team {
     __device__ __forceinline__ unsigned long long broken_joints() const {
         bool broken = false;
         if (has_joint()) {
-            const Joint k = joint<true>();
-            broken = k.angle < k.lo - kJointBreak || k.angle > k.hi + kJointBreak;
+            const float x = angle();
+            broken = x < ra.y - kJointBreak || x > ra.z + kJointBreak;
         }
         return (unsigned long long)(votes(broken) >> 1u);
     }
@@ -613,104 +599,80 @@ struct Team {
         return sum;
     }
 
-    // A pass over the bones in their order, each updating the values `own` of
-    // its two ends: `item(x0, x1)` on the pivot's and the node's. `table` is
-    // the shared table of the values.
+    // A pass over the bones in their order, each updating its two ends' values
+    // in `table`: `item(x0, x1)` on the pivot's and the node's.
     template <class F>
-    __device__ __forceinline__ void bones(float2& own, float2* table, F&& item) const {
-        if (in_order) {
-            float2 end = own, pivot = own;  // of this bone: after its turn
-            for (unsigned l = 1u; l <= levels; l++) {
-                const float2 pe = make_float2(from(end.x, prior), from(end.y, prior));
-                const float2 pp = make_float2(from(pivot.x, prior), from(pivot.y, prior));
-                if (level == l) {
-                    pivot = prior_pivot ? pp : pe;
-                    item(pivot, end);
-                }
+    __device__ __forceinline__ void bones(float2* table, F&& item) const {
+        float2& pivot = table[__float_as_uint(ba.x) & 31u];
+        for (unsigned l = 1u; l <= levels; l++) {
+            if (level == l) {
+                float2 x0 = pivot, x1 = table[i];
+                item(x0, x1);
+                pivot = x0;
+                table[i] = x1;
             }
-            const float2 x = make_float2(from(pivot.x, last), from(pivot.y, last));
-            own = has_last ? x : end;
-        } else {
-            // A pivot after its bone's end: one bone at a time.
-            if (has_node()) table[i] = own;
             __syncwarp();
-            for (unsigned j = 1u; j < T; j++) {
-                if (i == j && has_bone()) {
-                    float2 x0 = table[__float_as_uint(ba.x)], x1 = table[i];
-                    item(x0, x1);
-                    table[__float_as_uint(ba.x)] = x0;
-                    table[i] = x1;
-                }
-                __syncwarp();
-            }
-            if (has_node()) own = table[i];
         }
     }
 
-    // One substep (Creature::substep).
+    // One substep (Creature::substep). The positions and velocities are in
+    // shared memory at its start and end.
     __device__ __forceinline__ void substep() {
         const float2 pulls = muscles();
+        const bool node = has_node();
+        const float2 start = node ? pos(i) : make_float2(0.0f, 0.0f);
         // Drag.
         typename P::Wet wet{0.0f, 0.0f, 0.0f};
         if (f.w.has(CE_FLAG_WATER)) {
             const unsigned pivot = has_bone() ? __float_as_uint(ba.x) : 0u;
-            const float2 p0 = make_float2(from(p.x, pivot), from(p.y, pivot));
             const float r0 = from(nr.z, pivot);
             if (has_bone()) {
-                wet = f.wet_at(ba, r0, nr.z, p0, p);
+                wet = f.wet_at(ba, r0, nr.z, pos(pivot), start);
             }
         }
-        __syncwarp();
-        bones(v, &vel(0u), [&](float2& v0, float2& v1) { f.drag_at(bb, wet, v0, v1); });
+        bones(&vel(0u), [&](float2& v0, float2& v1) { f.drag_at(bb, wet, v0, v1); });
         // World forces, velocities and predicted positions.
-        const float2 start = p;
-        float4 s = make_float4(p.x, p.y, v.x, v.y);
-        f.integrate_at(i, nr, pulls, s);
-        p = make_float2(s.x, s.y);
-        bones(p, &pos(0u), [&](float2& p0, float2& p1) { P::bone_at(ba, p0, p1); });
-        // Joint ranges.
-        if (has_node()) pos(i) = p;
+        if (node) {
+            const float2 v = vel(i);
+            float4 s = make_float4(start.x, start.y, v.x, v.y);
+            f.integrate_at(i, nr, pulls, s);
+            pos(i) = make_float2(s.x, s.y);
+        }
         __syncwarp();
-        bool open = has_joint(), moved = false;
+        bones(&pos(0u), [&](float2& p0, float2& p1) { P::bone_at(ba, p0, p1); });
+        // Joint ranges.
+        bool open = has_joint();
         for (;;) {
-            Joint k;
-            float error = 0.0f;
-            if (open) {
-                k = joint<true>();
-                error = P::joint_error(k);
-            }
             // A NaN angle gives no error, as in the serial pass.
-            const unsigned past = votes(error != 0.0f);
-            if (!__any_sync(kFull, past != 0u)) {
+            const float error = open ? joint_error() : 0.0f;
+            const unsigned past = __ballot_sync(kFull, error != 0.0f);
+            if (past == 0u) {
                 break;
             }
-            moved = true;
-            __syncwarp();
-            if (open && (before & past) == 0u) {
+            if (open && (before & (past >> base)) == 0u) {
                 if (error != 0.0f) {
+                    const Joint k = joint();
                     const float wgt = P::joint_weight(k);
                     if (wgt > 0.0f) {
-                        push<false>(k, -error / wgt);
+                        push(k, -error / wgt, &pos(0u));
                     }
                 }
                 open = false;
             }
             __syncwarp();
         }
-        if (moved && has_node()) p = pos(i);
         // Ground contact and the velocity of the move.
-        float depth, back;
-        if (f.ground_at(nr, p, start, depth, back)) {
-            if (RECORD) {
-                shown_force.x += nr.x * depth * C::inv_h * C::inv_h;
-                shown_force.y += nr.x * back * C::inv_h * C::inv_h;
+        if (node) {
+            float2 p = pos(i);
+            float depth, back;
+            if (f.ground_at(nr, p, start, depth, back)) {
+                if (RECORD) {
+                    shown_force.x += nr.x * depth * C::inv_h * C::inv_h;
+                    shown_force.y += nr.x * back * C::inv_h * C::inv_h;
+                }
             }
-        }
-        v = make_float2((p.x - start.x) * C::inv_h, (p.y - start.y) * C::inv_h);
-        __syncwarp();
-        if (has_node()) {
             pos(i) = p;
-            vel(i) = v;
+            vel(i) = make_float2((p.x - start.x) * C::inv_h, (p.y - start.y) * C::inv_h);
         }
         __syncwarp();
         // Damping.
@@ -718,19 +680,18 @@ struct Team {
         Joint k;
         float wgt = 0.0f;
         if (has_joint()) {
-            k = joint<false>();
+            k = joint();
             wgt = P::joint_weight(k);
         }
         for (unsigned l = 1u; l <= damp_levels; l++) {
             if (damp_level == l) {
                 const float rate = P::joint_rate(k, vel(k.tip), vel(k.far), vel(k.hub));
                 if (wgt > 0.0f) {
-                    push<true>(k, __fmul_rn(-share, rate) / wgt);
+                    push(k, __fmul_rn(-share, rate) / wgt, &vel(0u));
                 }
             }
             __syncwarp();
         }
-        if (has_node()) v = vel(i);
     }
 
     // What score() reads and writes, for the team's first lane.
@@ -780,7 +741,8 @@ struct Team {
         // node order on the first.
         const bool broken = broken_joints() != 0ull;
         const bool node = has_node();
-        const bool failed = votes(node && !(fabsf(p.x) <= 1e6f && fabsf(p.y) <= 1e6f)) != 0u;
+        const float2 p = node ? pos(i) : make_float2(0.0f, 0.0f);
+        const bool failed = votes(!(fabsf(p.x) <= 1e6f && fabsf(p.y) <= 1e6f)) != 0u;
         bool touches = false, lifts = false;
         if (node && f.w.has(CE_FLAG_GROUND)) {
             const float2 g = ground_tally(f.w, p.x, r.amp, r.qphase, f.p);

@@ -110,9 +110,8 @@ struct Physics {
     struct Joint {
         unsigned tip, far, hub;
         float2 g_tip, g_far, g_hub;
-        float angle, lo, hi, w_tip, w_far, w_hub;
+        float w_tip, w_far, w_hub;
     };
-    template <bool LIMIT>
     __device__ __forceinline__ static Joint joint_at(unsigned j, const float4& ra, const float4& rb, const float2& pt,
                                                      const float2& pp, const float2& ct, const float2& ch) {
         Joint k;
@@ -121,8 +120,6 @@ struct Physics {
         k.hub = topo & 31u;
         k.far = (topo >> 15u) & 31u;
         const bool at_head = ((topo >> 20u) & 1u) != 0u;
-        k.lo = ra.y;
-        k.hi = ra.z;
         k.w_tip = rb.x;
         k.w_far = rb.y;
         k.w_hub = rb.z;
@@ -130,12 +127,6 @@ struct Physics {
         const float2 v = make_float2(ct.x - ch.x, ct.y - ch.y);
         const float uu = fmaxf(sum2(u.x, u.x, u.y, u.y), 1e-12f);
         const float vv = fmaxf(sum2(v.x, v.x, v.y, v.y), 1e-12f);
-        k.angle = 0.0f;
-        if (LIMIT) {
-            const float turn = atan2f(sum2(u.x, v.y, -u.y, v.x), sum2(u.x, v.x, u.y, v.y));
-            const float mid = ra.w;
-            k.angle = __fadd_rn(mid, wrap_of(__fsub_rn(turn, mid)));
-        }
         k.g_tip = make_float2(-v.y / vv, v.x / vv);
         const float2 g_u = make_float2(-u.y / uu, u.x / uu);
         k.g_far = at_head ? make_float2(-g_u.x, -g_u.y) : g_u;
@@ -148,16 +139,13 @@ struct Physics {
         const float hub = sum2(k.g_hub.x, k.g_hub.x, k.g_hub.y, k.g_hub.y);
         return __fmaf_rn(k.w_hub, hub, sum2(k.w_far, far, k.w_tip, tip));
     }
-    // How far joint k is past its range (0 within it).
-    __device__ __forceinline__ static float joint_error(const Joint& k) {
-        float error = 0.0f;
-        if (k.angle < k.lo) {
-            error = k.angle - k.lo;
-        }
-        if (k.angle > k.hi) {
-            error = k.angle - k.hi;
-        }
-        return error;
+    // The joint's angle, the turn from its range's middle.
+    __device__ __forceinline__ static float angle_at(const float4& ra, const float2& pt, const float2& pp,
+                                                     const float2& ct, const float2& ch) {
+        const float2 u = make_float2(pt.x - pp.x, pt.y - pp.y);
+        const float2 v = make_float2(ct.x - ch.x, ct.y - ch.y);
+        const float turn = atan2f(sum2(u.x, v.y, -u.y, v.x), sum2(u.x, v.x, u.y, v.y));
+        return __fadd_rn(ra.w, wrap_of(__fsub_rn(turn, ra.w)));
     }
     // The damping's relative turning speed at joint k.
     __device__ __forceinline__ static float joint_rate(const Joint& k, const float2& vt, const float2& vf,
