@@ -969,8 +969,8 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
         cudaGetLastError();
         per_sm = 1;
     }
-    const size_t needed = (t->count + cek::kBlock - 1) / cek::kBlock;
-    const unsigned grid = (unsigned)std::max<size_t>(1, std::min(needed, (size_t)per_sm * t->engine->sms));
+    const cek::AdjointGrid ag = cek::adjoint_grid(t->count, (size_t)t->engine->sms, (size_t)per_sm * t->engine->sms);
+    const unsigned grid = ag.grid;
     const size_t slot_b = cek::adjoint_slot_bytes(grid, t->rows, t->mm);
     const size_t grads_b = t->count * per * 4;
     if ((s = t->d_scratch.ensure(slot_b)) || (s = t->d_tape.ensure(cek::adjoint_tape_bytes(grid, t->rows, t->mm))) ||
@@ -990,6 +990,7 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
     CE_TRY(cek::launch_bucket(static_cast<const uint4*>(t->d_heads.ptr), 0u, (uint32_t)t->count, bk, st),
            "bucketing launch");
     cek::KernelArgs a = tape_args(t, bk);
+    a.lanes = ag.lanes;
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
     cek::LaunchSpec ls{t->rows, t->mm, t->flags, false, t->rate, grid, cek::kBlock, st};
     CE_TRY(cek::launch_adjoint(ls, a, t->params, static_cast<float4*>(t->d_tape.ptr),
@@ -1254,8 +1255,8 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         cudaGetLastError();
         per_sm = 1;
     }
-    const unsigned bgrid =
-        (unsigned)std::max<size_t>(1, std::min((n + cek::kBlock - 1) / cek::kBlock, (size_t)per_sm * e->sms));
+    const cek::AdjointGrid ag = cek::adjoint_grid(n, (size_t)e->sms, (size_t)per_sm * e->sms);
+    const unsigned bgrid = ag.grid;
     const size_t per_grad = cek::grad_floats(a->rows, a->mm);
     const size_t res_b = n * sizeof(ce_result);
     auto up = [&](DeviceBuf& d, const void* src, size_t bytes) -> ce_status {
@@ -1306,6 +1307,7 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         k.rows = a->rows;
         k.mm = a->mm;
         k.chunk_k = e->chunk_k;
+        k.lanes = ag.lanes;
         k.ckpt = static_cast<float*>(a->d_ckpt.ptr);
         k.ends = static_cast<uint32_t*>(a->d_ends.ptr);
         return k;
