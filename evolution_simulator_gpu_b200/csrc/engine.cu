@@ -198,6 +198,7 @@ std::vector<unsigned> class_grids(ce_engine* e, const std::vector<ClassPlan>& pl
 // 108; effects 131,072 149 / 211 and 262,144 283 / 233). A caller that sets
 // the blocks an SM asks for the lane kernel's launch shape and gets it.
 constexpr size_t kTeamMost = 24576;
+constexpr unsigned kTailMost = 24576;
 bool team_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamMost; }
 
 ce_status check_world(const ce_world* w) {
@@ -283,6 +284,116 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
             c.work += work_n[n];
         }
         if (c.count) plans.push_back(c);
+    }
+    return CE_OK;
+}
+
+// How a batch runs: each size class on teams of lanes or one creature a lane,
+// with the lane slots and the tail of each class in one scratch area.
+struct LaunchPlan {
+    std::vector<ClassPlan> classes;
+    std::vector<char> team;
+    std::vector<unsigned> grids;             // of the lane launches
+    std::vector<size_t> slots_at, tail_at;   // offsets in the scratch
+    size_t scratch = 0;
+    unsigned tail = 0;
+};
+
+// Creatures left at which a lane launch hands its trials over to teams.
+unsigned tail_most(const ce_engine* e, size_t count) {
+    return e->ctas_per_sm == 0 && count > kTeamMost ? kTailMost : 0u;
+}
+
+ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, int rate, LaunchPlan& lp) {
+    lp = LaunchPlan{};
+    ce_status s = plan_classes(pack, lp.classes, e->small_body);
+    if (s != CE_OK || lp.classes.empty()) return s;
+    if (team_pays(e, pack->count)) {
+        // One launch serves every node count.
+        ClassPlan all = lp.classes[0];
+        for (const ClassPlan& c : lp.classes) {
+            all.last_n = c.last_n;
+            all.rows = std::max(all.rows, c.rows);
+            all.mm = std::max(all.mm, c.mm);
+        }
+        all.count = (uint32_t)pack->count;
+        lp.classes.assign(1, all);
+    }
+    const size_t n = lp.classes.size();
+    bool any_team = false;
+    for (const ClassPlan& c : lp.classes) {
+        lp.team.push_back(team_pays(e, c.count) ? 1 : 0);
+        any_team = any_team || lp.team.back();
+    }
+    lp.grids.assign(n, 0u);
+    if (!any_team) {
+        lp.grids = class_grids(e, lp.classes, flags, rate);
+    }
+    lp.tail = tail_most(e, pack->count);
+    lp.slots_at.assign(n, 0);
+    lp.tail_at.assign(n, 0);
+    for (size_t c = 0; c < n; c++) {
+        if (lp.team[c]) continue;
+        const ClassPlan& k = lp.classes[c];
+        if (any_team) lp.grids[c] = grid_for(e, k.rows, k.mm, flags, false, rate, k.count);
+        lp.slots_at[c] = lp.scratch;
+        lp.scratch += (scratch_bytes(lp.grids[c], k.rows, k.mm, false) + 255u) & ~(size_t)255u;
+        lp.tail_at[c] = lp.scratch;
+        if (lp.tail) lp.scratch += cek::tail_bytes(k.rows, k.mm, lp.tail);
+    }
+    return CE_OK;
+}
+
+// A lane launch, and after it a team launch for the creatures it hands over.
+ce_status launch_lanes(ce_engine* e, const cek::LaunchSpec& ls, cek::KernelArgs a, const ce_params& p, void* tail,
+                       unsigned most) {
+    if (most) {
+        a.tail = cek::tail_layout(tail, most);
+        CE_TRY(cudaMemsetAsync(a.tail.counters, 0, cek::kTailCounters * 4u, ls.stream), "cudaMemsetAsync");
+    }
+    CE_TRY(cek::launch_advance(ls, a, p), "advance launch");
+    if (most) {
+        a.resume = 1u;
+        a.counter = a.tail.counters + cek::kTailClaimed;
+        const cek::TeamSpec ts{ls.flags, ls.rate, cek::team_blocks(a.rows, most), (unsigned)e->sms, ls.stream};
+        CE_TRY(cek::launch_team(ts, a, p), "tail launch");
+    }
+    return CE_OK;
+}
+
+// Runs a bucketed batch whose arrays are in `a`: the first class on `st`, the
+// second on `side`, which starts where `st` is and which the caller joins.
+ce_status launch_classes(ce_engine* e, const LaunchPlan& lp, cek::KernelArgs a, const cek::Buckets& bk, void* scratch,
+                         uint32_t flags, int rate, const ce_params& p, cudaStream_t st, cudaStream_t side) {
+    const size_t n = lp.classes.size();
+    a.order = bk.order;
+    a.chunk_k = e->chunk_k;
+    // Teams first: they leave room for the lanes' blocks, of which more start
+    // as the teams' ones end.
+    for (int lanes = 0; lanes < 2; lanes++) {
+        for (size_t c = 0; c < n; c++) {
+            if ((lp.team[c] != 0) != (lanes == 0)) continue;
+            const ClassPlan& k = lp.classes[c];
+            a.counter = bk.counters + k.first_n;
+            a.bounds = bk.bounds + k.first_n;
+            a.work = bk.work + k.first_n;
+            a.first_n = k.first_n;
+            a.queues = k.last_n - k.first_n + 1u;
+            a.count = k.count;
+            a.rows = k.rows;
+            a.mm = k.mm;
+            const cudaStream_t on = c == 0 ? st : side;
+            if (lanes == 0) {
+                const cek::TeamSpec ts{flags, rate, cek::team_blocks(a.rows, a.count), (unsigned)e->sms, on,
+                                       n > 1 ? 2u : 1u};
+                CE_TRY(cek::launch_team(ts, a, p), "advance launch");
+                continue;
+            }
+            a.scratch = reinterpret_cast<float4*>(static_cast<char*>(scratch) + lp.slots_at[c]);
+            const cek::LaunchSpec ls{k.rows, k.mm, flags, false, rate, lp.grids[c], cek::kBlock, on};
+            const ce_status s = launch_lanes(e, ls, a, p, static_cast<char*>(scratch) + lp.tail_at[c], lp.tail);
+            if (s != CE_OK) return s;
+        }
     }
     return CE_OK;
 }
@@ -448,27 +559,17 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
     }
     Slot& sl = e->slots[si];
     CE_TRY(cudaSetDevice(e->device), "cudaSetDevice");
-    std::vector<ClassPlan> plans;
-    if ((s = plan_classes(pack, plans, e->small_body)) != CE_OK) return s;
     const uint32_t flags = ce_world_flags(w);
     const int rate = (int)ce::world_rate(*w);
     ce_params p;
     ce_make_params(w, 0, (uint32_t)pack->count, 0, &p);
-    // Grids and scratch of the classes, which run side by side, each with its
-    // own part of the slot's scratch.
-    const bool team = team_pays(e, pack->count);
-    const std::vector<unsigned> grids = team ? std::vector<unsigned>(plans.size()) : class_grids(e, plans, flags, rate);
-    std::vector<size_t> scratch_at(plans.size());
-    size_t scratch = 0;
-    for (size_t c = 0; c < plans.size() && !team; c++) {
-        scratch_at[c] = scratch;
-        scratch += (scratch_bytes(grids[c], plans[c].rows, plans[c].mm, false) + 255u) & ~(size_t)255u;
-    }
+    LaunchPlan lp;
+    if ((s = plan_launch(e, pack, flags, rate, lp)) != CE_OK) return s;
     const size_t lanes_b = pack->lanes_len * 4, mus_b = pack->muscles_len * 4, heads_b = pack->count * 32;
     const size_t res_b = pack->count * sizeof(ce_result);
     if ((s = sl.d_lanes.ensure(lanes_b)) || (s = sl.d_muscles.ensure(mus_b)) || (s = sl.d_heads.ensure(heads_b)) ||
         (s = sl.d_buckets.ensure(cek::bucket_bytes(pack->count))) || (s = sl.d_results.ensure(res_b)) ||
-        (s = sl.d_scratch.ensure(scratch)) || (s = sl.h_upload.ensure(lanes_b + mus_b + heads_b)) ||
+        (s = sl.d_scratch.ensure(lp.scratch)) || (s = sl.h_upload.ensure(lanes_b + mus_b + heads_b)) ||
         (s = sl.h_results.ensure(res_b))) {
         return s;
     }
@@ -484,46 +585,12 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
            "bucketing launch");
     CE_TRY(cudaEventRecord(sl.bucketed, st), "cudaEventRecord");
     CE_TRY(cudaStreamWaitEvent(sl.side, sl.bucketed, 0), "cudaStreamWaitEvent");
-    if (team) {
-        // One launch serves every node count.
-        ClassPlan all = plans.empty() ? ClassPlan{} : plans[0];
-        for (const ClassPlan& c : plans) {
-            all.last_n = std::max(all.last_n, c.last_n);
-            all.rows = std::max(all.rows, c.rows);
-            all.mm = std::max(all.mm, c.mm);
-        }
-        if (!plans.empty()) all.count = (uint32_t)pack->count;
-        plans.resize(std::min<size_t>(plans.size(), 1), all);
-        if (!plans.empty()) plans[0] = all;
-    }
-    for (size_t c = 0; c < plans.size(); c++) {
-        cek::KernelArgs a{};
-        a.records = static_cast<const uint32_t*>(sl.d_lanes.ptr);
-        a.muscles = static_cast<const float*>(sl.d_muscles.ptr);
-        a.heads = static_cast<const uint4*>(sl.d_heads.ptr);
-        a.results = static_cast<ce_result*>(sl.d_results.ptr);
-        a.counter = bk.counters + plans[c].first_n;
-        a.first_n = plans[c].first_n;
-        a.scratch = reinterpret_cast<float4*>(static_cast<char*>(sl.d_scratch.ptr) + scratch_at[c]);
-        a.frames = nullptr;
-        a.order = bk.order;
-        a.bounds = bk.bounds + plans[c].first_n;
-        a.work = bk.work + plans[c].first_n;
-        a.queues = plans[c].last_n - plans[c].first_n + 1u;
-        a.count = plans[c].count;
-        a.rows = plans[c].rows;
-        a.mm = plans[c].mm;
-        a.frames_per_creature = 0;
-        a.chunk_k = e->chunk_k;
-        if (team) {
-            const cek::TeamSpec ts{flags, rate, cek::team_blocks(a.rows, a.count), (unsigned)e->sms, st};
-            CE_TRY(cek::launch_team(ts, a, p), "advance launch");
-            continue;
-        }
-        cek::LaunchSpec ls{plans[c].rows, plans[c].mm, flags, false, rate, grids[c], cek::kBlock,
-                           c == 0 ? st : sl.side};
-        CE_TRY(cek::launch_advance(ls, a, p), "advance launch");
-    }
+    cek::KernelArgs a{};
+    a.records = static_cast<const uint32_t*>(sl.d_lanes.ptr);
+    a.muscles = static_cast<const float*>(sl.d_muscles.ptr);
+    a.heads = static_cast<const uint4*>(sl.d_heads.ptr);
+    a.results = static_cast<ce_result*>(sl.d_results.ptr);
+    if ((s = launch_classes(e, lp, a, bk, sl.d_scratch.ptr, flags, rate, p, st, sl.side)) != CE_OK) return s;
     CE_TRY(cudaEventRecord(sl.joined, sl.side), "cudaEventRecord");
     CE_TRY(cudaStreamWaitEvent(st, sl.joined, 0), "cudaStreamWaitEvent");
     CE_TRY(cudaEventRecord(sl.stop, st), "cudaEventRecord");
@@ -688,7 +755,9 @@ extern "C" size_t ce_advance_scratch_bytes(ce_engine* e, uint32_t world_flags, u
                                            uint32_t max_muscles, uint32_t count) {
     if (!e || max_nodes < 2 || max_nodes > CE_MAX_NODES || max_muscles > CE_MAX_MUSCLES) return 0;
     if (rate != 60 && rate != 120) return 0;
-    return slots_part(e, world_flags, rate, max_nodes, max_muscles) + cek::bucket_bytes(count);
+    const unsigned most = tail_most(e, count);
+    return slots_part(e, world_flags, rate, max_nodes, max_muscles) + cek::bucket_bytes(count) +
+           (most ? cek::tail_bytes(max_nodes, max_muscles, most) : 0);
 }
 
 namespace {
@@ -742,9 +811,10 @@ ce_status advance_device(ce_engine* e, const uint32_t* records, const float* mus
         CE_TRY(cek::launch_team(ts, a, *params), "advance launch");
         return CE_OK;
     }
-    cek::LaunchSpec ls{max_nodes, max_muscles, world_flags, false, (int)rate, grid, cek::kBlock, st};
-    CE_TRY(cek::launch_advance(ls, a, *params), "advance launch");
-    return CE_OK;
+    const cek::LaunchSpec ls{max_nodes, max_muscles, world_flags, false, (int)rate, grid, cek::kBlock, st};
+    char* const tail = static_cast<char*>(scratch) + slots_part(e, world_flags, rate, max_nodes, max_muscles) +
+                       cek::bucket_bytes(params->count);
+    return launch_lanes(e, ls, a, *params, tail, tail_most(e, params->count));
 }
 }  // namespace
 
@@ -1475,10 +1545,9 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
     const uint32_t flags = ce_world_flags(w);
     const int rate = (int)ce::world_rate(*w);
     ce_params p;
-    // Plans, grids and scratch of every generation; one scratch a class.
-    std::vector<std::vector<ClassPlan>> plans(generations);
-    std::vector<std::vector<unsigned>> grids(generations);
-    size_t scratch_need[2] = {0, 0};
+    // Plans of every generation; they share one scratch.
+    std::vector<LaunchPlan> plans(generations);
+    size_t scratch_need = 0;
     g->gens.resize(generations);
     for (uint32_t k = 0; k < generations; k++) {
         const ce_wave_pack* pack = packs + k;
@@ -1486,15 +1555,8 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
             set_error("ce_graph_open: empty generation");
             return fail(CE_ERR_INVALID);
         }
-        if ((s = plan_classes(pack, plans[k], e->small_body)) != CE_OK) return fail(s);
-        const std::vector<unsigned> kg = class_grids(e, plans[k], flags, rate);
-        for (size_t ci = 0; ci < plans[k].size(); ci++) {
-            const ClassPlan& c = plans[k][ci];
-            const unsigned grid = kg[ci];
-            grids[k].push_back(grid);
-            const size_t at = grids[k].size() - 1;
-            scratch_need[at] = std::max(scratch_need[at], scratch_bytes(grid, c.rows, c.mm, false));
-        }
+        if ((s = plan_launch(e, pack, flags, rate, plans[k])) != CE_OK) return fail(s);
+        scratch_need = std::max(scratch_need, plans[k].scratch);
         ce_graph::Gen& gen = g->gens[k];
         gen.count = pack->count;
         const size_t lanes_b = pack->lanes_len * 4, mus_b = pack->muscles_len * 4, heads_b = pack->count * 32;
@@ -1509,10 +1571,8 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
             return fail(s);
         }
     }
-    g->scratch.resize(2);
-    for (int c = 0; c < 2; c++) {
-        if (scratch_need[c] && (s = g->scratch[c].ensure(scratch_need[c])) != CE_OK) return fail(s);
-    }
+    g->scratch.resize(1);
+    if (scratch_need && (s = g->scratch[0].ensure(scratch_need)) != CE_OK) return fail(s);
     g->events.resize(2 * generations, nullptr);
     for (auto& ev : g->events) {
         if ((s = cuda_status(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate"))) return fail(s);
@@ -1531,26 +1591,13 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
                           "bucketing launch");
         if (cap == CE_OK) cap = cuda_status(cudaEventRecord(g->events[2 * k], g->stream), "cudaEventRecord");
         if (cap == CE_OK) cap = cuda_status(cudaStreamWaitEvent(g->side, g->events[2 * k], 0), "cudaStreamWaitEvent");
-        for (size_t c = 0; c < plans[k].size() && cap == CE_OK; c++) {
-            cek::KernelArgs a{};
-            a.records = static_cast<const uint32_t*>(gen.lanes.ptr);
-            a.muscles = static_cast<const float*>(gen.muscles.ptr);
-            a.heads = static_cast<const uint4*>(gen.heads.ptr);
-            a.results = static_cast<ce_result*>(gen.results.ptr);
-            a.counter = bk.counters + plans[k][c].first_n;
-            a.scratch = static_cast<float4*>(g->scratch[c].ptr);
-            a.order = bk.order;
-            a.bounds = bk.bounds + plans[k][c].first_n;
-            a.work = bk.work + plans[k][c].first_n;
-            a.queues = plans[k][c].last_n - plans[k][c].first_n + 1u;
-            a.count = plans[k][c].count;
-            a.rows = plans[k][c].rows;
-            a.mm = plans[k][c].mm;
-            a.chunk_k = e->chunk_k;
-            cek::LaunchSpec ls{plans[k][c].rows, plans[k][c].mm, flags, false, rate, grids[k][c], cek::kBlock,
-                               c == 0 ? g->stream : g->side};
-            cap = cuda_status(cek::launch_advance(ls, a, p), "advance launch");
-        }
+        cek::KernelArgs a{};
+        a.records = static_cast<const uint32_t*>(gen.lanes.ptr);
+        a.muscles = static_cast<const float*>(gen.muscles.ptr);
+        a.heads = static_cast<const uint4*>(gen.heads.ptr);
+        a.results = static_cast<ce_result*>(gen.results.ptr);
+        if (cap == CE_OK)
+            cap = launch_classes(e, plans[k], a, bk, g->scratch[0].ptr, flags, rate, p, g->stream, g->side);
         if (cap == CE_OK) cap = cuda_status(cudaEventRecord(g->events[2 * k + 1], g->side), "cudaEventRecord");
         if (cap == CE_OK) cap = cuda_status(cudaStreamWaitEvent(g->stream, g->events[2 * k + 1], 0), "cudaStreamWaitEvent");
     }
@@ -1562,8 +1609,10 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
     // The largest tables of any launch in the graph.
     unsigned max_rows = 2, max_mm = 0;
     size_t max_smem = 0;
-    for (const auto& ps : plans) {
-        for (const ClassPlan& c : ps) {
+    for (const LaunchPlan& lp : plans) {
+        for (size_t ci = 0; ci < lp.classes.size(); ci++) {
+            if (lp.team[ci]) continue;
+            const ClassPlan& c = lp.classes[ci];
             const size_t b = cek::smem_bytes(c.rows, c.mm, cek::kBlock);
             if (b > max_smem) {
                 max_smem = b;

@@ -41,6 +41,24 @@ inline size_t smem_bytes(unsigned rows, unsigned mm, unsigned block) {
 constexpr unsigned kQueues = CE_MAX_NODES + 1u;  // node counts 0..32
 constexpr unsigned kBucketTile = 4096u;          // creatures a block buckets
 
+// The tail of a launch of one creature a lane. Once at most `most` of its
+// creatures are left, each lane writes its creature's state down at the end
+// of a step, and a team launch (team.cuh) finishes them: a creature takes a
+// team a third to a seventh of the time, and the launch's last creatures
+// leave most of its lanes idle.
+struct Tail {
+    uint32_t* counters;  // creatures done, states written, written for each of the three team sizes, claimed of each
+    uint32_t* order;     // states of each team size: `most` places each
+    float* state;        // tail_floats(rows, mm) each
+    uint32_t most;       // 0: no hand-over
+};
+constexpr unsigned kTailDone = 0, kTailStates = 1, kTailWritten = 2, kTailClaimed = 5, kTailCounters = 8;
+// Positions and velocities, energy stores and touchdown offsets, the 32 lane
+// words, the packed index and the next step.
+__host__ __device__ inline unsigned tail_floats(unsigned rows, unsigned mm) { return 4u * rows + 2u * mm + 34u; }
+size_t tail_bytes(unsigned rows, unsigned mm, unsigned most);
+Tail tail_layout(void* area, unsigned most);
+
 struct KernelArgs {
     const uint32_t* records;
     const float* muscles;
@@ -63,6 +81,8 @@ struct KernelArgs {
     float* ckpt;                   // CKPT: checkpoints, creature-minor: float f of checkpoint k of
                                    // creature c (packed index) at (k * checkpoint_floats + f) * count + c
     uint32_t* ends;                // CKPT: steps each creature's trial ran (packed index)
+    Tail tail;                     // plain kernel: where it hands over
+    uint32_t resume;               // team kernel: take the creatures of `tail` instead of the queues'
     // Niche epilogue at the result store (plain kernel; `cells` NULL: none):
     // each creature's metrics row (`metrics` may be NULL) and dense cell,
     // from its result, node count and shape class (packed index).
@@ -158,6 +178,7 @@ struct TeamSpec {
     int rate;
     unsigned blocks, sms;
     cudaStream_t stream;
+    unsigned share = 1u;  // leave the rest of the GPU to another launch: 1 / share of the blocks that fit
 };
 unsigned team_blocks(unsigned rows, size_t count);
 cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params& p);

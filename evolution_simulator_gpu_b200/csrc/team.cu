@@ -16,4 +16,25 @@ unsigned team_blocks(unsigned rows, size_t count) {
     return (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
 }
 
+namespace {
+size_t align256(size_t b) { return (b + 255u) & ~(size_t)255u; }
+}  // namespace
+
+size_t tail_bytes(unsigned rows, unsigned mm, unsigned most) {
+    return align256(kTailCounters * 4u) + align256((size_t)3u * most * 4u) +
+           align256((size_t)most * tail_floats(rows, mm) * 4u);
+}
+
+Tail tail_layout(void* area, unsigned most) {
+    char* p = static_cast<char*>(area);
+    Tail t;
+    t.counters = reinterpret_cast<uint32_t*>(p);
+    p += align256(kTailCounters * 4u);
+    t.order = reinterpret_cast<uint32_t*>(p);
+    p += align256((size_t)3u * most * 4u);
+    t.state = reinterpret_cast<float*>(p);
+    t.most = most;
+    return t;
+}
+
 }  // namespace cek

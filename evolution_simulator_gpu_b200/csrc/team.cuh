@@ -69,6 +69,14 @@ struct TeamClaim {
     bool drained = true;
 
     __device__ __forceinline__ unsigned queues() const { return a.queues > 0u ? a.queues : 1u; }
+    // The positions of queue q: the launch's queues, or the states of a tail
+    // by team size.
+    __device__ __forceinline__ unsigned start(unsigned q) const {
+        return a.resume ? q * a.tail.most : a.queues > 0u ? a.bounds[q] : 0u;
+    }
+    __device__ __forceinline__ unsigned size(unsigned q) const {
+        return a.resume ? a.tail.counters[kTailWritten + q] : a.queues > 0u ? a.bounds[q + 1u] - a.bounds[q] : a.count;
+    }
     // Queues of team size g: node counts up to 8, 16, 32.
     __device__ __forceinline__ unsigned first_queue(unsigned g) const {
         const unsigned n = g == 0u ? 0u : g == 1u ? 9u : g == 2u ? 17u : CE_MAX_NODES + 1u;
@@ -76,7 +84,11 @@ struct TeamClaim {
     }
     __device__ __forceinline__ void enter(unsigned g) {
         group = g;
-        if (a.queues == 0u) {
+        if (a.resume) {
+            lanes = 8u << g;
+            q_lo = g;
+            q_hi = g + 1u;
+        } else if (a.queues == 0u) {
             lanes = team_lanes(a.rows);
             q_lo = 0u;
             q_hi = 1u;
@@ -89,7 +101,7 @@ struct TeamClaim {
     }
     // The next team size with work; false when all have been served.
     __device__ __forceinline__ bool next_group() {
-        if (a.queues == 0u) return false;
+        if (a.queues == 0u && !a.resume) return false;
         if (++tried >= 3u) return false;
         enter(group == 2u ? 0u : group + 1u);
         return true;
@@ -97,7 +109,7 @@ struct TeamClaim {
 
     __device__ __forceinline__ TeamClaim(const KernelArgs& args, unsigned lane_, unsigned warp, unsigned warps)
         : a(args), lane(lane_), warps_total(warps) {
-        if (a.queues == 0u) {
+        if (a.queues == 0u && !a.resume) {
             enter(0u);
             return;
         }
@@ -107,10 +119,15 @@ struct TeamClaim {
         unsigned long long need[3], load[3], needs = 0ull, loads = 0ull;
 #pragma unroll
         for (unsigned g = 0u; g < 3u; g++) {
-            const unsigned q0 = first_queue(g), q1 = first_queue(g + 1u);
             const unsigned per = 4u >> g;
-            need[g] = (a.bounds[q1] - a.bounds[q0] + per - 1u) / per;
-            load[g] = (a.work[q1] - a.work[q0]) * (8ull << g);
+            if (a.resume) {
+                need[g] = (size(g) + per - 1u) / per;
+                load[g] = need[g];
+            } else {
+                const unsigned q0 = first_queue(g), q1 = first_queue(g + 1u);
+                need[g] = (a.bounds[q1] - a.bounds[q0] + per - 1u) / per;
+                load[g] = (a.work[q1] - a.work[q0]) * (8ull << g);
+            }
             needs += need[g];
             loads += load[g];
         }
@@ -137,8 +154,7 @@ struct TeamClaim {
                 unsigned c0 = kNone, c1 = 0u;
                 if (lane == 0u) {
                     for (unsigned q = q_hi; q-- > q_lo;) {
-                        const unsigned lo = a.queues > 0u ? a.bounds[q] : 0u;
-                        const unsigned n = (a.queues > 0u ? a.bounds[q + 1u] : a.count) - lo;
+                        const unsigned lo = start(q), n = size(q);
                         const unsigned seen = *reinterpret_cast<volatile unsigned*>(a.counter + q);
                         if (seen >= n) {
                             continue;
@@ -355,6 +371,10 @@ struct Team {
             }
         }
         __syncwarp();
+        if (!RECORD && !CKPT && a.resume != 0u) {
+            resume(fresh, slot);
+            __syncwarp();
+        }
         // The node's forces in muscle order: a muscle acts on a0 and a1 with
         // 1 - anchor_a and anchor_a, on b0 and b1 with minus the same of
         // anchor_b. A weight of zero adds a zero, which changes no sum but
@@ -416,6 +436,31 @@ struct Team {
                 record_frame(t, fresh);
             }
         }
+    }
+
+    // The state that a lane wrote down (Trial::hand_over) over the start's.
+    __device__ __forceinline__ const float* tail_state(unsigned slot) const {
+        return a.tail.state + (size_t)slot * tail_floats(a.rows, a.mm);
+    }
+    __device__ __forceinline__ void resume(bool fresh, unsigned slot) {
+        if (!fresh) {
+            return;
+        }
+        const float* s = tail_state(slot);
+        if (has_node()) {
+            pos(i) = make_float2(s[4u * i], s[4u * i + 1u]);
+            vel(i) = make_float2(s[4u * i + 2u], s[4u * i + 3u]);
+        }
+        s += 4u * a.rows;
+        for (unsigned k = i; k < r.muscles; k += T) {
+            store(k).x = s[2u * k];
+            offset(k) = s[2u * k + 1u];
+        }
+        s += 2u * a.mm;
+        for (unsigned q = i; q < 32u; q += T) {
+            words()[q] = s[q];
+        }
+        r.step = __float_as_uint(s[33]);
     }
 
     // Calls `put(weight)` for each weight of muscle k that acts on node i, in
@@ -819,8 +864,14 @@ __global__ void __launch_bounds__(kTeamBlock, kTeamMinBlocks) team_kernel(const 
         const unsigned mine = __shfl_sync(kFull, got, t.base);
         const bool fresh = !live && mine != kNone;
         if (__any_sync(kFull, fresh)) {
-            const unsigned cidx = fresh ? (a.order ? __ldg(a.order + mine) : p.base + mine) : 0u;
-            t.begin(fresh, cidx, mine);
+            unsigned cidx = 0u, slot = mine;
+            if (fresh && a.resume != 0u) {
+                slot = a.tail.order[mine];
+                cidx = __float_as_uint(t.tail_state(slot)[4u * a.rows + 2u * a.mm + 32u]);
+            } else if (fresh) {
+                cidx = a.order ? __ldg(a.order + mine) : p.base + mine;
+            }
+            t.begin(fresh, cidx, slot);
             live = live || fresh;
         }
         if (!__any_sync(kFull, live)) {

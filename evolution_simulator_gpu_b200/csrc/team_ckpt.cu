@@ -6,8 +6,8 @@ namespace cek {
 
 cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_params& p) {
     const auto go = [&](auto w) -> cudaError_t {
-        if (s.rate == 60) return team_one<decltype(w), false, 60, true>(w, s.blocks, s.sms, a, p, s.stream);
-        if (s.rate == 120) return team_one<decltype(w), false, 120, true>(w, s.blocks, s.sms, a, p, s.stream);
+        if (s.rate == 60) return team_one<decltype(w), false, 60, true>(w, s, a, p);
+        if (s.rate == 120) return team_one<decltype(w), false, 120, true>(w, s, a, p);
         return cudaErrorInvalidValue;
     };
     switch (s.flags) {

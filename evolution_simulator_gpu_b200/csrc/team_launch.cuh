@@ -11,7 +11,8 @@ namespace cek {
 inline unsigned team_warp_bytes(const KernelArgs& a, bool record) {
     unsigned most = 0u;
     for (unsigned lanes = 8u; lanes <= 32u; lanes *= 2u) {
-        const bool used = a.queues == 0u ? lanes == team_lanes(a.rows)
+        const bool used = a.resume ? lanes <= team_lanes(a.rows)
+                          : a.queues == 0u ? lanes == team_lanes(a.rows)
                                          : lanes >= team_lanes(a.first_n) && lanes <= team_lanes(a.rows);
         const unsigned bytes = 32u / lanes * TeamLayout::make(lanes, a.mm, record).bytes;
         if (used && bytes > most) most = bytes;
@@ -28,25 +29,25 @@ cudaError_t team_occupancy_one(unsigned warp_bytes, int* blocks) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kern, (int)kTeamBlock, smem);
 }
 
-// Launches the kernel on as many blocks as fit, at most `blocks`.
+// Launches the kernel on as many blocks as fit.
 template <class W, bool RECORD, int RATE, bool CKPT>
-cudaError_t team_one(const W& w, unsigned blocks, unsigned sms, const KernelArgs& a, const ce_params& p,
-                     cudaStream_t stream) {
+cudaError_t team_one(const W& w, const TeamSpec& s, const KernelArgs& a, const ce_params& p) {
     const unsigned warp_bytes = team_warp_bytes(a, RECORD);
     int per_sm = 0;
     const cudaError_t e = team_occupancy_one<W, RECORD, RATE, CKPT>(warp_bytes, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const unsigned grid = blocks < (unsigned)per_sm * sms ? blocks : (unsigned)per_sm * sms;
+    if (s.share > 1u && per_sm > 1) per_sm = (per_sm + (int)s.share - 1) / (int)s.share;
+    const unsigned grid = s.blocks < (unsigned)per_sm * s.sms ? s.blocks : (unsigned)per_sm * s.sms;
     team_kernel<W, RECORD, RATE, CKPT>
-        <<<grid > 0u ? grid : 1u, kTeamBlock, (size_t)warp_bytes * (kTeamBlock / 32u), stream>>>(a, p, w, warp_bytes);
+        <<<grid > 0u ? grid : 1u, kTeamBlock, (size_t)warp_bytes * (kTeamBlock / 32u), s.stream>>>(a, p, w, warp_bytes);
     return cudaGetLastError();
 }
 
 template <bool RECORD, int RATE>
 cudaError_t team_in_world(const TeamSpec& s, const KernelArgs& a, const ce_params& p) {
     const auto go = [&](auto w) {
-        return team_one<decltype(w), RECORD, RATE, false>(w, s.blocks, s.sms, a, p, s.stream);
+        return team_one<decltype(w), RECORD, RATE, false>(w, s, a, p);
     };
     switch (s.flags) {
         case kWorldCalm: return go(StaticWorld<kWorldCalm>{});

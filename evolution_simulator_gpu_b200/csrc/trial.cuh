@@ -525,6 +525,35 @@ struct Trial {
         }
     };
 
+    // Writes this lane's creature down for a team launch to go on with.
+    __device__ __forceinline__ static void hand_over(const Body& b, const KernelArgs& a) {
+        const LaneRegs& r = b.r;
+        const unsigned slot = atomicAdd(a.tail.counters + kTailStates, 1u);
+        const unsigned g = r.nodes <= 8u ? 0u : r.nodes <= 16u ? 1u : 2u;
+        a.tail.order[g * a.tail.most + atomicAdd(a.tail.counters + kTailWritten + g, 1u)] = slot;
+        float* s = a.tail.state + (size_t)slot * tail_floats(a.rows, a.mm);
+        for (unsigned i = 0u; i < r.nodes; i++) {
+            const float2 q = b.t.pos(i), v = b.t.vel(i);
+            s[4u * i] = q.x;
+            s[4u * i + 1u] = q.y;
+            s[4u * i + 2u] = v.x;
+            s[4u * i + 3u] = v.y;
+        }
+        s += 4u * a.rows;
+        for (unsigned k = 0u; k < r.muscles; k++) {
+            s[2u * k] = b.t.muscle(k).x;
+            s[2u * k + 1u] = b.L.word_cold(b.S.muscle + 5u * k + kMState, 2);
+        }
+        s += 2u * a.mm;
+        float lw[32];
+        Words{b}.load(lw);
+        for (unsigned q = 0u; q < 32u; q++) {
+            s[q] = lw[q];
+        }
+        s[32] = __uint_as_float(r.cidx);
+        s[33] = __uint_as_float(r.step);
+    }
+
     // One step of the creature on this lane (shaders/creature.cu:956-1248).
     // Returns whether the lane still has a creature.
     __device__ __forceinline__ static bool step(const Body& b, const KernelArgs& a) {
@@ -685,8 +714,26 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) advance_kernel(const Kerne
         if (__ballot_sync(kFull, live) == 0u) {
             break;
         }
+        const bool was = live;
         if (live) {
             live = T::step(b, a);
+        }
+        if (!RECORD && !CKPT && a.tail.most != 0u) {
+            const unsigned ended = __ballot_sync(kFull, was && !live);
+            unsigned done = 0u;
+            if (lane == 0u) {
+                if (ended != 0u) {
+                    atomicAdd(a.tail.counters + kTailDone, (unsigned)__popc(ended));
+                }
+                done = *reinterpret_cast<volatile unsigned*>(a.tail.counters + kTailDone);
+            }
+            done = __shfl_sync(kFull, done, 0);
+            if (a.count - done <= a.tail.most) {
+                if (live) {
+                    T::hand_over(b, a);
+                    live = false;
+                }
+            }
         }
     }
 }
