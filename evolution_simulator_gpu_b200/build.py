@@ -35,7 +35,8 @@ NVCC_FLAGS = [
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-fopenmp"]
 
 CUDA_SOURCES = ["advance.cu", "adjoint.cu", "bucket.cu", "engine.cu", "metrics.cu", "peak.cu", "noalloc.cu",
-                "sample.cu", "pack.cu", "cma.cu", "audit.cu", "team.cu", "team_record.cu", "team_ckpt.cu"]
+                "sample.cu", "pack.cu", "cma.cu", "audit.cu", "team.cu", "team_record.cu", "team_ckpt.cu",
+                "team_adjoint.cu"]
 # The device packer, gene gradients and ascent step, the CMA-ES emitters and
 # the rung audit's sums round as their host counterparts: IEEE division and
 # square root, no contraction of multiply-adds.

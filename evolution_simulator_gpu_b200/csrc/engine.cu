@@ -201,6 +201,10 @@ constexpr size_t kTeamMost = 24576;
 constexpr unsigned kTailMost = 24576;
 bool team_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamMost; }
 
+// Whether a backward run of `count` creatures goes on teams.
+constexpr size_t kTeamBackMost = 65536;
+bool team_back_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamBackMost; }
+
 ce_status check_world(const ce_world* w) {
     if (!w) {
         set_error("null world");
@@ -1041,9 +1045,17 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
     }
     const cek::AdjointGrid ag = cek::adjoint_grid(t->count, (size_t)t->engine->sms, (size_t)per_sm * t->engine->sms);
     const unsigned grid = ag.grid;
-    const size_t slot_b = cek::adjoint_slot_bytes(grid, t->rows, t->mm);
+    const bool team = team_back_pays(t->engine, t->count);
+    unsigned blocks = 0;
+    if (team) {
+        CE_TRY(cek::team_adjoint_blocks(t->rows, t->mm, t->flags, t->rate, (unsigned)t->engine->sms, t->count, &blocks),
+               "backward launch");
+    }
+    const size_t slot_b = team ? 0 : cek::adjoint_slot_bytes(grid, t->rows, t->mm);
+    const size_t tape_b = team ? cek::team_adjoint_tape_bytes(blocks, t->rows, t->mm)
+                               : cek::adjoint_tape_bytes(grid, t->rows, t->mm);
     const size_t grads_b = t->count * per * 4;
-    if ((s = t->d_scratch.ensure(slot_b)) || (s = t->d_tape.ensure(cek::adjoint_tape_bytes(grid, t->rows, t->mm))) ||
+    if ((s = t->d_scratch.ensure(slot_b)) || (s = t->d_tape.ensure(tape_b)) ||
         (s = t->d_grads.ensure(grads_b)) || (s = t->d_weights.ensure(t->count * 4)) ||
         (mismatches && (s = t->d_mismatch.ensure(t->count * 4)))) {
         return s;
@@ -1062,12 +1074,19 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
     cek::KernelArgs a = tape_args(t, bk);
     a.lanes = ag.lanes;
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
-    cek::LaunchSpec ls{t->rows, t->mm, t->flags, false, t->rate, grid, cek::kBlock, st};
-    CE_TRY(cek::launch_adjoint(ls, a, t->params, static_cast<float4*>(t->d_tape.ptr),
-                               static_cast<float*>(t->d_grads.ptr),
-                               dl_dfitness ? static_cast<const float*>(t->d_weights.ptr) : nullptr,
-                               mismatches ? static_cast<uint32_t*>(t->d_mismatch.ptr) : nullptr),
-           "backward launch");
+    const float* weights = dl_dfitness ? static_cast<const float*>(t->d_weights.ptr) : nullptr;
+    uint32_t* mismatch = mismatches ? static_cast<uint32_t*>(t->d_mismatch.ptr) : nullptr;
+    if (team) {
+        const cek::TeamSpec ts{t->flags, t->rate, blocks, (unsigned)t->engine->sms, st};
+        CE_TRY(cek::launch_team_adjoint(ts, a, t->params, static_cast<float*>(t->d_tape.ptr),
+                                        static_cast<float*>(t->d_grads.ptr), weights, mismatch),
+               "backward launch");
+    } else {
+        cek::LaunchSpec ls{t->rows, t->mm, t->flags, false, t->rate, grid, cek::kBlock, st};
+        CE_TRY(cek::launch_adjoint(ls, a, t->params, static_cast<float4*>(t->d_tape.ptr),
+                                   static_cast<float*>(t->d_grads.ptr), weights, mismatch),
+               "backward launch");
+    }
     CE_TRY(cudaEventRecord(t->stop, st), "cudaEventRecord");
     if ((s = tape_time(t, &t->backward_seconds)) != CE_OK) return s;
     CE_TRY(cudaMemcpy(grads, t->d_grads.ptr, grads_b, cudaMemcpyDeviceToHost), "cudaMemcpy");
@@ -1327,6 +1346,12 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
     }
     const cek::AdjointGrid ag = cek::adjoint_grid(n, (size_t)e->sms, (size_t)per_sm * e->sms);
     const unsigned bgrid = ag.grid;
+    const bool team_back = team_back_pays(e, n);
+    unsigned bblocks = 0;
+    if (team_back && (s = cuda_status(cek::team_adjoint_blocks(a->rows, a->mm, flags, a->rate, (unsigned)e->sms, n, &bblocks),
+                                      "backward launch")) != CE_OK) {
+        return fail(s);
+    }
     const size_t per_grad = cek::grad_floats(a->rows, a->mm);
     const size_t res_b = n * sizeof(ce_result);
     auto up = [&](DeviceBuf& d, const void* src, size_t bytes) -> ce_status {
@@ -1346,8 +1371,9 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         (s = a->d_ckpt.ensure(n * (size_t)a->ckpts * cek::checkpoint_floats(a->rows, a->mm) * 4)) ||
         (s = a->d_ends.ensure(n * 4)) ||
         (s = a->d_scratch.ensure(std::max(scratch_bytes(fgrid, a->rows, a->mm, false),
-                                          cek::adjoint_slot_bytes(bgrid, a->rows, a->mm)))) ||
-        (s = a->d_tape.ensure(cek::adjoint_tape_bytes(bgrid, a->rows, a->mm))) ||
+                                          team_back ? 0 : cek::adjoint_slot_bytes(bgrid, a->rows, a->mm)))) ||
+        (s = a->d_tape.ensure(team_back ? cek::team_adjoint_tape_bytes(bblocks, a->rows, a->mm)
+                                        : cek::adjoint_tape_bytes(bgrid, a->rows, a->mm))) ||
         (s = a->d_grads.ensure(n * per_grad * 4)) || (s = a->d_mg.ensure(std::max<size_t>(muscles_len, 1) * 5 * 8)) ||
         (s = a->d_ng.ensure(std::max<size_t>(nodes_len, 1) * 8))) {
         return fail(s);
@@ -1398,9 +1424,12 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
             ce = team_pays(e, n) ? cek::launch_team_ckpt(ts, ka, a->params) : cek::launch_forward_ckpt(fs, ka, a->params);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(a->d_grads.ptr, 0, n * per_grad * 4, st);
         if (ce == cudaSuccess) ce = cek::launch_bucket(heads_d, 0u, (uint32_t)n, bk, st);
+        const cek::TeamSpec tb{flags, a->rate, bblocks, (unsigned)e->sms, st};
         if (ce == cudaSuccess)
-            ce = cek::launch_adjoint(bs, ka, a->params, static_cast<float4*>(a->d_tape.ptr),
-                                     static_cast<float*>(a->d_grads.ptr), nullptr, nullptr);
+            ce = team_back ? cek::launch_team_adjoint(tb, ka, a->params, static_cast<float*>(a->d_tape.ptr),
+                                                      static_cast<float*>(a->d_grads.ptr), nullptr, nullptr)
+                           : cek::launch_adjoint(bs, ka, a->params, static_cast<float4*>(a->d_tape.ptr),
+                                                 static_cast<float*>(a->d_grads.ptr), nullptr, nullptr);
         if (ce == cudaSuccess)
             ce = cek::launch_gene_grads(dpop, static_cast<const float*>(a->d_trig.ptr),
                                         static_cast<const uint32_t*>(a->d_order.ptr), n, a->world,

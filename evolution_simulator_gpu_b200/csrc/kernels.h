@@ -185,6 +185,15 @@ cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params&
 cudaError_t launch_team_record(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 
+// The backward run on teams (team_adjoint.cu): its blocks, the bytes of its
+// segment tapes and its launch (TeamSpec::blocks of them).
+constexpr unsigned kTeamAdjointMinBlocks = 6;
+cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t count,
+                                unsigned* blocks);
+size_t team_adjoint_tape_bytes(unsigned blocks, unsigned rows, unsigned mm);
+cudaError_t launch_team_adjoint(const TeamSpec& s, const KernelArgs& a, const ce_params& p, float* tape, float* grads,
+                                const float* weights, uint32_t* mismatch);
+
 // 16-byte lines of one lane's slot.
 unsigned slot_lines(unsigned rows, unsigned mm, bool record);
 

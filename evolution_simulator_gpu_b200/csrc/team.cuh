@@ -236,13 +236,14 @@ struct Team {
     __device__ __forceinline__ unsigned from(unsigned x, unsigned n) const { return __shfl_sync(kFull, x, base + n); }
     __device__ __forceinline__ unsigned votes(bool x) const { return (__ballot_sync(kFull, x) >> base) & mask; }
 
-    __device__ __forceinline__ void place(unsigned lane, unsigned lanes, char* warp_mem) {
+    // `extra`: bytes of a creature's memory behind its own (a multiple of 128).
+    __device__ __forceinline__ void place(unsigned lane, unsigned lanes, char* warp_mem, unsigned extra = 0u) {
         T = lanes;
         i = lane & (T - 1u);
         base = lane - i;
         mask = T == 32u ? kFull : (1u << T) - 1u;
         S = TeamLayout::make(T, a.mm, RECORD);
-        mem = warp_mem + (base / T) * S.bytes;
+        mem = warp_mem + (base / T) * (S.bytes + extra);
         nr = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
         ba = bb = ra = rb = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         shown_force = make_float2(0.0f, 0.0f);
@@ -660,10 +661,29 @@ struct Team {
         }
     }
 
+    // What the reverse of a substep reads of this lane's node, bone and joint:
+    // the values that each sequential pass saw, the muscles' force and the
+    // contact.
+    struct Kept {
+        float2 pulls, landing;           // muscle force; position before the ground pass
+        float2 drag0, drag1, bone0, bone1;  // the bone's ends before its drag and its projection
+        float2 pt, pp, ct, ch;           // positions that the joint's push saw
+        float2 vt, vf, vh;               // velocities that its damping saw
+        Joint k;                         // its damping's gradients and
+        float wgt;                       // their weight
+        bool pushed, touched, slid;
+    };
+
     // One substep (Creature::substep). The positions and velocities are in
-    // shared memory at its start and end.
-    __device__ __forceinline__ void substep() {
+    // shared memory at its start and end. `KEEP`: what the reverse reads goes
+    // to `kept`.
+    template <bool KEEP = false>
+    __device__ __forceinline__ void substep(Kept* kept = nullptr) {
         const float2 pulls = muscles();
+        if (KEEP) {
+            kept->pulls = pulls;
+            kept->pushed = kept->touched = kept->slid = false;
+        }
         const bool node = has_node();
         const float2 start = node ? pos(i) : make_float2(0.0f, 0.0f);
         // Drag.
@@ -675,7 +695,13 @@ struct Team {
                 wet = f.wet_at(ba, r0, nr.z, pos(pivot), start);
             }
         }
-        bones(&vel(0u), [&](float2& v0, float2& v1) { f.drag_at(bb, wet, v0, v1); });
+        bones(&vel(0u), [&](float2& v0, float2& v1) {
+            if (KEEP) {
+                kept->drag0 = v0;
+                kept->drag1 = v1;
+            }
+            f.drag_at(bb, wet, v0, v1);
+        });
         // World forces, velocities and predicted positions.
         if (node) {
             const float2 v = vel(i);
@@ -684,7 +710,13 @@ struct Team {
             pos(i) = make_float2(s.x, s.y);
         }
         __syncwarp();
-        bones(&pos(0u), [&](float2& p0, float2& p1) { P::bone_at(ba, p0, p1); });
+        bones(&pos(0u), [&](float2& p0, float2& p1) {
+            if (KEEP) {
+                kept->bone0 = p0;
+                kept->bone1 = p1;
+            }
+            P::bone_at(ba, p0, p1);
+        });
         // Joint ranges.
         bool open = has_joint();
         for (;;) {
@@ -699,6 +731,14 @@ struct Team {
                     const Joint k = joint();
                     const float wgt = P::joint_weight(k);
                     if (wgt > 0.0f) {
+                        if (KEEP) {
+                            const unsigned topo = __float_as_uint(ra.x);
+                            kept->pushed = true;
+                            kept->pt = pos((topo >> 5u) & 31u);
+                            kept->pp = pos((topo >> 10u) & 31u);
+                            kept->ct = pos(i);
+                            kept->ch = pos(topo & 31u);
+                        }
                         push(k, -error / wgt, &pos(0u));
                     }
                 }
@@ -710,7 +750,15 @@ struct Team {
         if (node) {
             float2 p = pos(i);
             float depth, back;
-            if (f.ground_at(nr, p, start, depth, back)) {
+            bool slid;
+            if (KEEP) {
+                kept->landing = p;
+            }
+            if (f.ground_at(nr, p, start, depth, back, slid)) {
+                if (KEEP) {
+                    kept->touched = true;
+                    kept->slid = slid;
+                }
                 if (RECORD) {
                     shown_force.x += nr.x * depth * C::inv_h * C::inv_h;
                     shown_force.y += nr.x * back * C::inv_h * C::inv_h;
@@ -730,12 +778,22 @@ struct Team {
         }
         for (unsigned l = 1u; l <= damp_levels; l++) {
             if (damp_level == l) {
-                const float rate = P::joint_rate(k, vel(k.tip), vel(k.far), vel(k.hub));
+                const float2 vt = vel(k.tip), vf = vel(k.far), vh = vel(k.hub);
+                if (KEEP) {
+                    kept->vt = vt;
+                    kept->vf = vf;
+                    kept->vh = vh;
+                }
+                const float rate = P::joint_rate(k, vt, vf, vh);
                 if (wgt > 0.0f) {
                     push(k, __fmul_rn(-share, rate) / wgt, &vel(0u));
                 }
             }
             __syncwarp();
+        }
+        if (KEEP) {
+            kept->k = k;
+            kept->wgt = wgt;
         }
     }
 

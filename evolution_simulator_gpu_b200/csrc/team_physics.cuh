@@ -21,7 +21,8 @@ __device__ __forceinline__ float sum2(float a, float b, float c, float d) {
 }
 
 // Ground height and slope under x (shaders/creature.cu:166-226).
-template <class W>
+// `BACK`: as the backward run's contact fuses it.
+template <bool BACK = false, class W>
 __device__ __forceinline__ float2 ground_of(const W& w, float x, float amp, float qphase, const ce_params& p) {
     float height = 0.0f, slope = 0.0f;
     if (w.has(CE_FLAG_TERRAIN)) {
@@ -36,7 +37,7 @@ __device__ __forceinline__ float2 ground_of(const W& w, float x, float amp, floa
             __fmul_rn(__fmul_rn(0.65f * 32.0f, w0), __fsub_rn(1.0f, __fmul_rn(2.0f, u0))), 1.0f / 1.1f,
             __fmul_rn(__fmul_rn(0.35f * 32.0f, w1), __fsub_rn(1.0f, __fmul_rn(2.0f, u1))), 1.0f / 0.43f);
         if (w.has(CE_FLAG_SLOPE)) {
-            height = sum2(p.slope, x, amp, bumps);
+            height = BACK ? sum2(amp, bumps, p.slope, x) : sum2(p.slope, x, amp, bumps);
             slope = W::fixed ? __fmaf_rn(amp, rise, p.slope) : __fadd_rn(__fmul_rn(amp, rise), p.slope);
         } else {
             height = __fmul_rn(amp, bumps);
@@ -300,10 +301,11 @@ struct Physics {
 
     // Ground contact and friction of a node (shaders/creature.cu:640-679).
     // `q` is the node's position (moved when it touches) and `f0` its
-    // position at the start of the substep. Returns whether it touches, and
-    // the push out of the ground and back along it (a recording's forces).
-    __device__ __forceinline__ bool ground_at(const float4& nr, float2& q, const float2& f0, float& depth,
-                                              float& back) const {
+    // position at the start of the substep. Returns whether it touches, the
+    // push out of the ground and back along it (a recording's forces), and
+    // whether it slid.
+    __device__ __forceinline__ bool ground_at(const float4& nr, float2& q, const float2& f0, float& depth, float& back,
+                                              bool& slid) const {
         if (!w.has(CE_FLAG_GROUND)) {
             return false;
         }
@@ -330,7 +332,8 @@ struct Physics {
         const float tx = ny, ty = -nx;
         const float slide = sum2(q.x - f0.x, tx, q.y - f0.y, ty);
         const float budget = __fmul_rn(mu, depth);
-        back = fabsf(slide) <= budget ? slide : copysignf(budget, slide);
+        slid = !(fabsf(slide) <= budget);
+        back = slid ? copysignf(budget, slide) : slide;
         q.x = __fmaf_rn(-tx, back, q.x);
         q.y = __fmaf_rn(-ty, back, q.y);
         return true;
