@@ -1214,7 +1214,8 @@ __global__ void __launch_bounds__(kBlock, 2) adjoint_kernel(const KernelArgs a, 
 // schedulers without a warp spreads over all of them, a few lanes in each:
 // 1,021 creatures x 10 s of the refined search's world 1,024 -> 657 ms. With a
 // warp on every scheduler full warps are better (16,381 calm creatures x 4 s:
-// 360 ms, and 375 ms as two half-filled warps a scheduler).
+// 360 ms, and 375 ms as two half-filled warps a scheduler). Batches as small
+// as that run here where the caller set the blocks an SM; others go on teams.
 AdjointGrid adjoint_grid(size_t count, size_t sms, size_t blocks) {
     constexpr size_t per = kBlock / 32u;
     const size_t lanes = (count + sms * per - 1u) / (sms * per);

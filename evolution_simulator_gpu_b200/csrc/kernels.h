@@ -187,7 +187,7 @@ cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_pa
 
 // The backward run on teams (team_adjoint.cu): its blocks, the bytes of its
 // segment tapes and its launch (TeamSpec::blocks of them).
-constexpr unsigned kTeamAdjointMinBlocks = 6;
+constexpr unsigned kTeamAdjointMinBlocks = 4;
 cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t count,
                                 unsigned* blocks);
 size_t team_adjoint_tape_bytes(unsigned blocks, unsigned rows, unsigned mm);

@@ -270,7 +270,7 @@ struct Team {
         const ce_params& pr = f.p;
         const uint32_t* rec = nullptr;
         const float* mus = nullptr;
-        float4 new_nr = nr, new_ba = ba, new_bb = bb, new_ra = ra, new_rb = rb;
+        [[maybe_unused]] float4 new_nr = nr, new_ba = ba, new_bb = bb, new_ra = ra, new_rb = rb;
         unsigned pivot = 0u;
         bool foot = false;
         if (fresh) {

@@ -11,6 +11,14 @@
 // stays in the lane's registers from the rerun to the reverse, so a substep
 // moves nothing but its tape entry, and every sum has the order of the serial
 // reverse.
+//
+// Bound by the chain of a creature's dependent operations where the launch
+// leaves schedulers idle, and by instruction issue above. Those values need
+// registers: 4 blocks of 64 threads an SM (255 registers) against 6 (168, with
+// spills) took 90 / 100 ms at 1,021 creatures of the refined search's world x
+// 4 s and 150 / 197 ms at 8,192; 5 blocks are 6% faster at 16,384 calm ones
+// and up to 25% slower in the other world. Backward before, on lanes: 268 and
+// 360 ms; 16,384 calm creatures x 2 s 191 -> 145 ms.
 #include <cuda_runtime.h>
 
 #include <type_traits>

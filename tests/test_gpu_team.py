@@ -132,3 +132,22 @@ def test_checkpoints_match(engine, lanes, world):
             k = (ended[c] + 15) // 16
             assert (ca[c, :k, cols] == cb[c, :k, cols]).all()
         assert (a.backward().view(np.uint32) == b.backward().view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("world", ["calm", "effects", "tremors"])
+@pytest.mark.parametrize("nodes,muscles,count", [(2, 1, 3), (3, 2, 33), (8, 24, 9), (9, 7, 13), (16, 40, 5),
+                                                 (17, 60, 3), (32, 24, 2)])
+def test_gradients_match(engine, lanes, world, nodes, muscles, count):
+    """Anchors and tendons, weighted, at 120 substeps a second; the rerun of
+    every segment must reproduce the forward run."""
+    w = ce.make_world(duration=1.5, rate=120, **WORLDS[world])
+    pop = evolved(bodies(nodes, muscles, count) if nodes > 2 else ce.generate(WORKLOADS["refine"].spec, count))
+    pop.muscles["sensor"] = 255
+    wave = ce.pack(pop, w)
+    weights = np.linspace(-2.0, 3.0, len(wave)).astype(np.float32)
+    with engine.forward(wave, w) as a, lanes.forward(wave, w) as b:
+        ga, bad = a.backward(weights, check=True)
+        gb, _ = b.backward(weights, check=True)
+    assert not bad.any()
+    assert np.isfinite(ga).all() and (ga != 0).any()
+    assert (ga.view(np.uint32) == gb.view(np.uint32)).all()
