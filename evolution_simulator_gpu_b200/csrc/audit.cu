@@ -7,10 +7,10 @@
 // features (src/rungs.rs:224-235), and class A's feature words are listed.
 //
 // The sums are order dependent in float64, so they are added in row order,
-// one thread a sum: the rows are first compacted in order (a count, a scan of
-// the tiles' counts and an ordered write), then a block walks them in chunks,
-// the chunk's features staged in shared memory, and each of its 172 threads
-// (2 rungs x 2 classes x (count, 6 sums, 36 products)) adds its own column.
+// one thread a sum: the rows are first compacted in order (a count and an
+// ordered write), then a block a (rung, class) walks them in chunks: 30 warps
+// stage the next chunk's features of its class while the first 43 threads add
+// one column each (a count, 6 sums, 36 products) of the last one.
 // Built with no fused multiply-adds, so every sum equals the reference's to
 // the bit.
 #include <cuda_runtime.h>
@@ -28,8 +28,11 @@ constexpr uint32_t kAudit = 1u, kExempt = 2u;  // rungs::AUDIT, rungs::EXEMPT (s
 constexpr unsigned kFeatures = 6u;
 constexpr unsigned kTile = 256u;                 // threads of the count and write kernels
 constexpr unsigned kColumns = 1u + kFeatures + kFeatures * kFeatures;  // count, sums, products: 43
-constexpr unsigned kGroup = 64u;                 // threads a (rung, class) group of the sum kernel
-constexpr unsigned kChunk = 4u * kGroup;         // rows staged at a time: one a thread
+constexpr unsigned kAdders = 64u;                // threads of a sum block that add: a column each
+constexpr unsigned kChunk = 960u;                // its others, which stage a row each
+constexpr unsigned kAhead = 8u;                  // rows whose products are formed ahead of the additions
+constexpr unsigned kStaged = (kChunk + kAhead) * (kFeatures + 1u);  // doubles; the last kAhead rows are read, not added
+constexpr size_t kSumBytes = 2u * kStaged * sizeof(double);
 
 __device__ __forceinline__ uint32_t bits(float f) { return __float_as_uint(f); }
 
@@ -99,82 +102,71 @@ __device__ __forceinline__ bool is_row(const Inputs& in, size_t i, const Trace& 
     return (in.genomes[i].flags & kAudit) != 0u && t.steps() != 0u;
 }
 
-// Audit::note's tallies and the audit rows of each block's tile.
+// Audit::note's tallies and the audit rows of each block's tile, added up over
+// the warp before they meet in shared memory (one 64-bit shared atomic a
+// thread and tally had most of the kernel's time: 43 -> 9 us at 300,007).
 __global__ void __launch_bounds__(kTile) audit_count_kernel(const Inputs in, uint32_t* tile_rows, ce_audit* out) {
-    __shared__ unsigned long long s_steps, s_stops[3];
-    __shared__ unsigned s_rows;
-    if (threadIdx.x == 0u) {
-        s_steps = 0ull;
-        s_stops[0] = s_stops[1] = s_stops[2] = 0ull;
-        s_rows = 0u;
-    }
-    __syncthreads();
+    __shared__ unsigned long long s_steps[kTile / 32u];
+    __shared__ unsigned s_counts[4][kTile / 32u];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const size_t lo = (size_t)blockIdx.x * in.tile, hi = min(lo + in.tile, in.count);
-    unsigned long long steps = 0ull, stops[3] = {0ull, 0ull, 0ull};
-    unsigned rows = 0u;
+    unsigned long long steps = 0ull;
+    unsigned counts[4] = {0u, 0u, 0u, 0u};  // stops, rows
     for (size_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
         const ce_result& r = in.results[i];
         const Trace t(r);
         steps += t.steps();
         if (r.screened > 0.0f) {
             const uint32_t k = t.stopped_by();
-            stops[k == 1u ? 0 : (k == 2u ? 1 : 2)] += 1ull;
+            counts[k == 1u ? 0 : (k == 2u ? 1 : 2)] += 1u;
         }
-        rows += is_row(in, i, t) ? 1u : 0u;
+        counts[3] += is_row(in, i, t) ? 1u : 0u;
     }
-    atomicAdd(&s_steps, steps);
-    for (int k = 0; k < 3; k++) atomicAdd(&s_stops[k], stops[k]);
-    atomicAdd(&s_rows, rows);
+    for (unsigned d = 16u; d > 0u; d >>= 1) steps += __shfl_down_sync(0xffffffffu, steps, d);
+#pragma unroll
+    for (unsigned q = 0u; q < 4u; q++) counts[q] = __reduce_add_sync(0xffffffffu, counts[q]);
+    if (lane == 0u) {
+        s_steps[warp] = steps;
+#pragma unroll
+        for (unsigned q = 0u; q < 4u; q++) s_counts[q][warp] = counts[q];
+    }
     __syncthreads();
-    if (threadIdx.x == 0u) {
-        tile_rows[blockIdx.x] = s_rows;
-        atomicAdd(reinterpret_cast<unsigned long long*>(&out->steps), s_steps);
-        for (int k = 0; k < 3; k++) atomicAdd(reinterpret_cast<unsigned long long*>(&out->stops[k]), s_stops[k]);
+    if (threadIdx.x < 5u) {
+        unsigned long long all = 0ull;
+        for (unsigned v = 0u; v < kTile / 32u; v++) {
+            all += threadIdx.x == 4u ? s_steps[v] : (unsigned long long)s_counts[threadIdx.x][v];
+        }
+        if (threadIdx.x == 3u) {
+            tile_rows[blockIdx.x] = (uint32_t)all;
+        } else if (all != 0ull) {
+            uint64_t* const to = threadIdx.x == 4u ? &out->steps : &out->stops[threadIdx.x];
+            atomicAdd(reinterpret_cast<unsigned long long*>(to), all);
+        }
     }
 }
 
-// Exclusive offsets of the tiles' rows and the batch's totals: one block of
-// 1024 threads, two tiles a thread (at most 2048 tiles).
-constexpr unsigned kMaxTiles = 2048u;
-__global__ void __launch_bounds__(1024) audit_scan_kernel(uint32_t* tile_rows, unsigned tiles, size_t count,
-                                                           ce_audit* out) {
-    __shared__ uint32_t warp_sum[32];
-    const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    const uint32_t x0 = 2u * t < tiles ? tile_rows[2u * t] : 0u, x1 = 2u * t + 1u < tiles ? tile_rows[2u * t + 1u] : 0u;
-    const uint32_t mine = x0 + x1;
-    uint32_t incl = mine;
-    for (unsigned d = 1u; d < 32u; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += y;
-    }
-    if (lane == 31u) warp_sum[warp] = incl;
-    __syncthreads();
-    if (warp == 0u) {
-        uint32_t w = warp_sum[lane], wi = w;
-        for (unsigned d = 1u; d < 32u; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, wi, d);
-            if (lane >= d) wi += y;
-        }
-        warp_sum[lane] = wi - w;  // exclusive
-        if (lane == 31u) {
-            out->rows = wi;
-            out->creatures = count;
-        }
-    }
-    __syncthreads();
-    const uint32_t before = warp_sum[warp] + incl - mine;
-    if (2u * t < tiles) tile_rows[2u * t] = before;
-    if (2u * t + 1u < tiles) tile_rows[2u * t + 1u] = before + x0;
-}
-
-// Each tile writes its rows' indices in order: a block-wide ordered
-// compaction, 256 creatures at a time.
+// Each tile writes its rows' indices in order, behind those of the tiles
+// before it, whose counts it adds up itself: a block-wide ordered compaction,
+// 256 creatures at a time. The last tile has the batch's totals.
 __global__ void __launch_bounds__(kTile) audit_write_kernel(const Inputs in, const uint32_t* tile_rows,
-                                                            uint32_t* row_index) {
+                                                            uint32_t* row_index, ce_audit* out) {
     __shared__ unsigned warp_rows[kTile / 32u];
     __shared__ unsigned base;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0u) base = tile_rows[blockIdx.x];
+    unsigned ahead = 0u;
+    for (unsigned k = threadIdx.x; k < blockIdx.x; k += blockDim.x) ahead += tile_rows[k];
+    ahead = __reduce_add_sync(0xffffffffu, ahead);
+    if (lane == 0u) warp_rows[warp] = ahead;
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+        unsigned all = 0u;
+        for (unsigned k = 0u; k < blockDim.x / 32u; k++) all += warp_rows[k];
+        base = all;
+        if (blockIdx.x + 1u == gridDim.x) {
+            out->rows = all + tile_rows[blockIdx.x];
+            out->creatures = in.count;
+        }
+    }
     const size_t lo = (size_t)blockIdx.x * in.tile, hi = min(lo + in.tile, in.count);
     for (size_t start = lo; start < hi; start += blockDim.x) {
         const size_t i = start + threadIdx.x;
@@ -195,98 +187,108 @@ __global__ void __launch_bounds__(kTile) audit_write_kernel(const Inputs in, con
     }
 }
 
-// GenAudit::of over the compacted rows, in order. Four groups of 64
-// threads, one a (rung, class): per chunk of 256 rows each row's features
-// are staged once as float64 (with a constant 1 in slot 6), each group gets
-// the chunk's rows of its class in row order, and thread c < 43 of a group
-// adds its column over them: c = 0 the count, 1-6 feature c - 1 times the
-// constant 1 (an exact product, so the sum is Sums::add's), 7-42 the product
-// of features (c - 7) / 6 and (c - 7) % 6. Every column is one row-ordered
-// chain of float64 multiply and add, with no branch on the row.
-__global__ void __launch_bounds__(kChunk) audit_sum_kernel(const Inputs in, const uint32_t* row_index, ce_audit* out,
-                                                           uint16_t* a_words, size_t a_cap) {
-    __shared__ double feat[kChunk][2][kFeatures + 1u];
-    __shared__ uint16_t list[4][kChunk];
-    __shared__ unsigned warp_count[4][kChunk / 32u], list_len[4];
-    const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    const unsigned group = t / kGroup, col = t % kGroup, r = group >> 1, k = group & 1u;
+// GenAudit::of over the compacted rows, in order, a block a (rung, class).
+// Each chunk's rows of the class are staged in row order as float64 with a
+// constant 1 behind their features, and thread c < 43 adds its column over
+// them: c = 0 the count, 1-6 feature c - 1 times the constant 1 (an exact
+// product, so the sum is Sums::add's), 7-42 the product of features
+// (c - 7) / 6 and (c - 7) % 6. Every column is one row-ordered chain of
+// float64 multiply and add, with no branch on the row.
+//
+// Bound by the gathers of a row (its index, then its result, genome and bar,
+// then its muscle) and by the chain of additions. One block for all four
+// groups that staged 256 rows, then added them, took 103 us for 2,344 rows;
+// 960 rows at a time, staged while the last ones are added, 50 us, and with
+// the next rows' products formed under the chain (8 cycles an addition, 19
+// with its loads in line) 25 us.
+__global__ void __launch_bounds__(kAdders + kChunk) audit_sum_kernel(const Inputs in, const uint32_t* row_index,
+                                                                     ce_audit* out, uint16_t* a_words, size_t a_cap) {
+    extern __shared__ double feat[];  // [2][kChunk + kAhead][kFeatures + 1]
+    __shared__ unsigned warp_count[kChunk / 32u], staged[2];
+    const unsigned r = blockIdx.x >> 1, k = blockIdx.x & 1u, lane = threadIdx.x & 31u;
+    const unsigned col = threadIdx.x;
     const unsigned fa = col == 0u ? kFeatures : (col <= kFeatures ? col - 1u : (col - 1u - kFeatures) / kFeatures);
     const unsigned fb = col <= kFeatures ? kFeatures : (col - 1u - kFeatures) % kFeatures;
     const uint32_t rows = out->rows;
+    const uint32_t chunks = rows / kChunk + (rows % kChunk ? 1u : 0u);
     double acc = 0.0;
     unsigned long long n = 0ull;
-    for (uint32_t start = 0u; start < rows; start += kChunk) {
-        const uint32_t len = min(kChunk, rows - start);
-        __syncthreads();  // the last chunk's lists and features are read
-        unsigned cls[2] = {2u, 2u};  // per rung: 0 class A, 1 class B, 2 neither
-        if (t < len) {
-            const uint32_t i = row_index[start + t];
-            const ce_result& res = in.results[i];
-            const Trace tr(res);
-            const ce_genome& g = in.genomes[i];
-            const float bar = in.bars[i];
-            const bool counted = (g.flags & kExempt) == 0u && isfinite(bar);
-            const bool pass3 = res.screen_x >= bar;
-            const float period = g.muscle_count > 0u ? in.muscles[g.muscle_start].period : 0.0f;
-            const float ph = half_to_float(float_to_half(period));
-            for (unsigned rr = 0u; rr < 2u; rr++) {
-                const float f[kFeatures] = {half_of(tr.w[rr / 2u], rr % 2u == 1u), half_of(tr.w[3], rr == 1u),
-                                            half_of(tr.w[4u + rr], false), half_of(tr.w[6], rr == 1u),
-                                            half_of(tr.w[4u + rr], true), ph};
+    uint32_t index = threadIdx.x >= kAdders && threadIdx.x - kAdders < rows ? row_index[threadIdx.x - kAdders] : 0u;
+    for (uint32_t c = 0u; c <= chunks; c++) {
+        if (threadIdx.x >= kAdders && c < chunks) {
+            const unsigned t = threadIdx.x - kAdders, warp = t >> 5;
+            const size_t row = (size_t)c * kChunk + t;
+            float f[kFeatures] = {};
+            bool mine = false;
+            if (row < rows) {
+                const uint32_t i = index;
+                if (row + kChunk < rows) index = row_index[row + kChunk];
+                const ce_result& res = in.results[i];
+                const Trace tr(res);
+                const ce_genome& g = in.genomes[i];
+                const float bar = in.bars[i];
+                const bool counted = (g.flags & kExempt) == 0u && isfinite(bar);
+                const float period = g.muscle_count > 0u ? in.muscles[g.muscle_start].period : 0.0f;
+                f[0] = half_of(tr.w[0], r == 1u);
+                f[1] = half_of(tr.w[3], r == 1u);
+                f[2] = half_of(r == 0u ? tr.w[4] : tr.w[5], false);
+                f[3] = half_of(tr.w[6], r == 1u);
+                f[4] = half_of(r == 0u ? tr.w[4] : tr.w[5], true);
+                f[5] = half_to_float(float_to_half(period));
                 bool finite = true;
 #pragma unroll
-                for (unsigned x = 0u; x < kFeatures; x++) {
-                    feat[t][rr][x] = (double)f[x];
-                    finite = finite && isfinite(f[x]);
-                }
-                feat[t][rr][kFeatures] = 1.0;
+                for (unsigned x = 0u; x < kFeatures; x++) finite = finite && isfinite(f[x]);
                 // rungs::RUNG_STEPS: R1 at step 60, R2 at 150.
-                cls[rr] = (counted && tr.steps() > (rr == 0u ? 60u : 150u) && finite) ? (pass3 ? 0u : 1u) : 2u;
+                mine = counted && tr.steps() > (r == 0u ? 60u : 150u) && finite && (res.screen_x >= bar) == (k == 0u);
             }
-        }
-        // Each group's rows in row order: a ballot a warp, then the warps'
-        // counts before this one.
-        unsigned ballot[4];
+            // The class's rows in row order: a ballot a warp, then the
+            // counts of the warps before.
+            const unsigned ballot = __ballot_sync(0xffffffffu, mine);
+            if (lane == 0u) warp_count[warp] = __popc(ballot);
+            asm volatile("bar.sync 1, %0;" ::"n"(kChunk) : "memory");
+            const unsigned have = lane < kChunk / 32u ? warp_count[lane] : 0u;
+            const unsigned all = __reduce_add_sync(0xffffffffu, have);
+            const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? have : 0u);
+            if (mine) {
+                const unsigned j = before + __popc(ballot & ((1u << lane) - 1u));
+                double* const to = feat + (c & 1u) * kStaged + j * (kFeatures + 1u);
 #pragma unroll
-        for (unsigned q = 0u; q < 4u; q++) {
-            ballot[q] = __ballot_sync(0xffffffffu, cls[q >> 1] == (q & 1u));
-            if (lane == 0u) warp_count[q][warp] = __popc(ballot[q]);
-        }
-        __syncthreads();
+                for (unsigned x = 0u; x < kFeatures; x++) to[x] = (double)f[x];
+                to[kFeatures] = 1.0;
+                if (k == 0u && a_words && n + j < a_cap) {  // class A's feature words
+                    uint16_t* const w = a_words + ((size_t)r * a_cap + n + j) * kFeatures;
 #pragma unroll
-        for (unsigned q = 0u; q < 4u; q++) {
-            if ((ballot[q] >> lane) & 1u) {
-                unsigned before = 0u;
-                for (unsigned v = 0u; v < warp; v++) before += warp_count[q][v];
-                list[q][before + __popc(ballot[q] & ((1u << lane) - 1u))] = (uint16_t)t;
-            }
-        }
-        if (t < 4u) {
-            unsigned all = 0u;
-            for (unsigned v = 0u; v < kChunk / 32u; v++) all += warp_count[t][v];
-            list_len[t] = all;
-        }
-        __syncthreads();
-        const unsigned L = list_len[group];
-        if (col < kColumns) {
-            if (col > 0u) {
-#pragma unroll 4
-                for (unsigned j = 0u; j < L; j++) {
-                    const unsigned q = list[group][j];
-                    acc += feat[q][r][fa] * feat[q][r][fb];
+                    for (unsigned x = 0u; x < kFeatures; x++) w[x] = (uint16_t)float_to_half(f[x]);
                 }
             }
-            if (k == 0u && a_words) {
-                // Class A's feature words, the group's threads sharing the rows.
-                for (unsigned j = col; j < L; j += kColumns) {
-                    if (n + j >= a_cap) break;
-                    const unsigned q = list[group][j];
-                    uint16_t* w = a_words + ((size_t)r * a_cap + n + j) * kFeatures;
-                    for (unsigned x = 0u; x < kFeatures; x++) w[x] = (uint16_t)float_to_half((float)feat[q][r][x]);
-                }
+            // Rows of zeros fill up the last kAhead: no sum is -0, so they add nothing.
+            if (t < kAhead && all + t < (all + kAhead - 1u) / kAhead * kAhead) {
+                double* const to = feat + (c & 1u) * kStaged + (all + t) * (kFeatures + 1u);
+#pragma unroll
+                for (unsigned x = 0u; x <= kFeatures; x++) to[x] = 0.0;
             }
+            if (t == 0u) staged[c & 1u] = all;
+            n += all;
+        } else if (col < kColumns && c > 0u) {
+            const unsigned len = staged[(c - 1u) & 1u];
+            const double* at = feat + ((c - 1u) & 1u) * kStaged;
+            double now[kAhead], next[kAhead];
+#pragma unroll
+            for (unsigned x = 0u; x < kAhead; x++) now[x] = at[x * (kFeatures + 1u) + fa] * at[x * (kFeatures + 1u) + fb];
+            for (unsigned j = 0u; j < len; j += kAhead) {
+                at += kAhead * (kFeatures + 1u);
+#pragma unroll
+                for (unsigned x = 0u; x < kAhead; x++) {
+                    next[x] = at[x * (kFeatures + 1u) + fa] * at[x * (kFeatures + 1u) + fb];
+                }
+#pragma unroll
+                for (unsigned x = 0u; x < kAhead; x++) acc += now[x];
+#pragma unroll
+                for (unsigned x = 0u; x < kAhead; x++) now[x] = next[x];
+            }
+            n += len;
         }
-        n += L;
+        __syncthreads();
     }
     if (col < kColumns) {
         ce_audit_sums& s = k == 0u ? out->a[r] : out->b[r];
@@ -330,10 +332,12 @@ extern "C" ce_status ce_audit_device(const ce_result* results, const ce_genome* 
     Inputs in{results, genomes, muscles, bars, count, (count + tiles - 1u) / tiles};
     if (in.tile == 0u) in.tile = 1u;
     audit_count_kernel<<<tiles, kTile, 0, st>>>(in, tile_rows, out);
-    audit_scan_kernel<<<1, 1024, 0, st>>>(tile_rows, tiles, count, out);
-    audit_write_kernel<<<tiles, kTile, 0, st>>>(in, tile_rows, row_index);
-    audit_sum_kernel<<<1, kChunk, 0, st>>>(in, row_index, out, a_words, a_cap);
-    e = cudaGetLastError();
+    audit_write_kernel<<<tiles, kTile, 0, st>>>(in, tile_rows, row_index, out);
+    e = cudaFuncSetAttribute(audit_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSumBytes);
+    if (e == cudaSuccess) {
+        audit_sum_kernel<<<4, kAdders + kChunk, kSumBytes, st>>>(in, row_index, out, a_words, a_cap);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) {
         ce::set_error(std::string("ce_audit_device: launch: ") + cudaGetErrorString(e));
         return CE_ERR_DEVICE;

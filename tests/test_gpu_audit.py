@@ -104,3 +104,22 @@ def test_audit_words_stop_at_the_callers_capacity(engine):
         for r in range(2):
             assert got["sums"][r][0][0] == sums[r][0][0]
             assert (got["a_words"][r] == a_rows[r][:cap]).all() and len(got["a_words"][r]) == cap
+
+
+@pytest.mark.parametrize("rows", [0, 1, 7, 8, 9, 959, 960, 961, 1921])
+@pytest.mark.parametrize("one_class", [False, True])
+def test_audit_at_the_edges_of_the_staged_rows(engine, rows, one_class):
+    """Around 8 and 960 rows, all of them of one class or of both."""
+    rng = np.random.default_rng(rows)
+    count = rows + 300
+    pop = ce.generate(WORKLOADS["game"].spec, count)
+    words = rng.integers(0, 1 << 32, size=(count, 7), dtype=np.uint64).astype(np.uint32) & np.uint32(0x7bff7bff)
+    words[:, 2] = (words[:, 2] & 0xffff) | np.uint32(600 << 16)
+    res = np.zeros(count, ce.RESULT_DTYPE)
+    for k, f in enumerate(A.TRACE_FIELDS):
+        res[f] = words[:, k].view(np.float32)
+    res["screen_x"] = 9.0 if one_class else rng.normal(2.0, 1.0, count).astype(np.float32)
+    flags = np.zeros(count, np.uint32)
+    flags[rng.permutation(count)[:rows]] = A.AUDIT
+    pop.genomes["flags"] = flags
+    assert check(res, pop, np.full(count, 2.0, np.float32))["rows"] == rows

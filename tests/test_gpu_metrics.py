@@ -46,3 +46,28 @@ def test_device_metrics_equal_host_metrics(engine, workload, screen):
         assert (cells >= 0).all()
     if screen:
         assert (host_m["screened"] > 0).any()
+
+
+@pytest.mark.parametrize("count", [1, 255, 256, 257, 1000])
+@pytest.mark.parametrize("rows", [True, False])
+def test_device_metrics_of_ragged_batches(engine, count, rows):
+    """Batches that end inside a block's 256 creatures; nothing is written
+    behind them, and the metrics may be left out."""
+    torch = pytest.importorskip("torch")
+    world = ce.make_world(duration=0.5)
+    pop = ce.generate(WORKLOADS["game"].spec, count)
+    wave = ce.pack(pop, world)
+    results, _ = engine.run(wave, world)
+    host_m = ce.to_metrics(results, (wave.heads[:, 0] & 255).astype(np.uint32), world)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_res, d_heads = up(results.view(np.float32).reshape(-1)), up(wave.heads.view(np.int32).reshape(-1))
+    d_shape = up(ce.shape_classes(pop, wave))
+    d_m = torch.full((9 * count + 64,), 77, dtype=torch.int32, device="cuda")
+    d_cells = torch.full((count + 8,), 77, dtype=torch.int64, device="cuda")
+    ce.metrics_device(d_res.data_ptr(), d_heads.data_ptr(), d_shape.data_ptr(), count, world,
+                      d_m.data_ptr() if rows else 0, d_cells.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    words, cells = d_m.cpu().numpy(), d_cells.cpu().numpy()
+    assert (words[:9 * count] == (host_m.view(np.int32).reshape(-1) if rows else 77)).all()
+    assert (words[9 * count:] == 77).all() and (cells[count:] == 77).all()
+    assert (cells[:count] == ce.niche_cells(pop, host_m, indices=wave.slots)).all()
