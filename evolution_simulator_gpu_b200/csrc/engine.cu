@@ -202,10 +202,10 @@ constexpr unsigned kTailMost = 24576;
 bool team_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamMost; }
 
 // Whether a backward run of `count` creatures goes on teams: the same trade
-// (ms on teams / on lanes: calm x 2 s 8,192 81 / 178, 16,384 145 / 191, 32,768
-// 264 / 204; the refined search's world x 4 s 16,384 243 / 479, 32,768 425 /
-// 532).
-constexpr size_t kTeamBackMost = 24576;
+// (ms on teams / on lanes: calm x 2 s 8,192 59 / 176, 16,384 107 / 188, 32,768
+// 195 / 206, 49,152 287 / 241; the refined search's world x 4 s 16,384 176 /
+// 473, 32,768 313 / 536, 65,536 594 / 725).
+constexpr size_t kTeamBackMost = 32768;
 bool team_back_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamBackMost; }
 
 ce_status check_world(const ce_world* w) {

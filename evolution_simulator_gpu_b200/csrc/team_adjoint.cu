@@ -7,18 +7,18 @@
 // and that bone's joint; the items of a pass run in levels from the end (an
 // item goes when every later item at its nodes has), the muscles go round the
 // lanes and each node's lane adds up its own in the muscles' order. What the
-// reverse reads of the substep (the values that each pass saw, the contact)
-// stays in the lane's registers from the rerun to the reverse, so a substep
-// moves nothing but its tape entry, and every sum has the order of the serial
-// reverse.
+// reverse reads of a substep (the values that each pass saw, the contact)
+// goes to the segment's tape as the rerun meets it, 9 float4 a lane, and is
+// fetched a substep ahead; every sum has the order of the serial reverse.
 //
 // Bound by the chain of a creature's dependent operations where the launch
-// leaves schedulers idle, and by instruction issue above. Those values need
-// registers: 4 blocks of 64 threads an SM (255 registers) against 6 (168, with
-// spills) took 90 / 100 ms at 1,021 creatures of the refined search's world x
-// 4 s and 150 / 197 ms at 8,192; 5 blocks are 6% faster at 16,384 calm ones
-// and up to 25% slower in the other world. Backward before, on lanes: 268 and
-// 360 ms; 16,384 calm creatures x 2 s 191 -> 145 ms.
+// leaves schedulers idle, and by instruction issue above; the tape's 300 B a
+// lane and substep are under a tenth of the memory's rate. Running each
+// substep again before its reverse, with those values in registers, moves 32 B
+// instead and took 92 ms against 68 at 1,021 creatures of the refined search's
+// world x 4 s, 152 / 110 ms at 8,192 and 144 / 107 ms at 16,384 calm ones x 2 s
+// (on lanes: 269, 366 and 188 ms). 4 blocks of 64 threads an SM have 255
+// registers; 5 and 6 (168, with spills) took 79 ms.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -47,10 +47,14 @@ struct TeamAdjointLayout {
     }
 };
 
-// A substep's entry in a team's segment tape: (x, y, vx, vy) a lane, then the
+// A substep's entry in a team's segment tape: float4s of every lane, its start
+// state (x, y, vx, vy) and what the reverse reads of the substep, then the
 // energy stores.
+enum TapePart : unsigned {
+    kTapeState, kTapePulls, kTapeDrag, kTapeBone, kTapeEnds, kTapeHub, kTapeTurn, kTapeParent, kTapeOwn, kTapeParts
+};
 __host__ __device__ inline unsigned team_tape_floats(unsigned lanes, unsigned mm) {
-    return 4u * lanes + ((mm + 3u) & ~3u);
+    return 4u * kTapeParts * lanes + ((mm + 3u) & ~3u);
 }
 __host__ __device__ inline unsigned team_tape_warp_floats(unsigned rows, unsigned mm) {
     unsigned most = 0u;
@@ -202,42 +206,107 @@ struct TeamBackward : Team<W, false, RATE, false> {
     }
 
     __device__ __forceinline__ float* tape_at(unsigned k) const { return tape + (size_t)k * team_tape_floats(T, a.mm); }
+    __device__ __forceinline__ float4& part(unsigned k, TapePart n) const {
+        return reinterpret_cast<float4*>(tape_at(k))[n * T + i];
+    }
+    __device__ __forceinline__ static float4 pair(float2 u, float2 v) { return make_float4(u.x, u.y, v.x, v.y); }
     __device__ __forceinline__ void save_state(unsigned k) const {
-        float* s = tape_at(k);
         if (has_node()) {
-            const float2 q = pos(i), u = vel(i);
-            reinterpret_cast<float4*>(s)[i] = make_float4(q.x, q.y, u.x, u.y);
+            part(k, kTapeState) = pair(pos(i), vel(i));
         }
+        float* s = tape_at(k) + 4u * kTapeParts * T;
         for (unsigned m = i; m < r.muscles; m += T) {
-            s[4u * T + m] = store(m).x;
+            s[m] = store(m).x;
         }
     }
     // A substep's start state, as registers hold it until put_state().
     __device__ __forceinline__ float4 state_of(unsigned k) const {
-        return has_node() ? reinterpret_cast<const float4*>(tape_at(k))[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return has_node() ? part(k, kTapeState) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     __device__ __forceinline__ void put_state(unsigned k, const float4& s) const {
         if (has_node()) {
             pos(i) = make_float2(s.x, s.y);
             vel(i) = make_float2(s.z, s.w);
         }
+        const float* e = tape_at(k) + 4u * kTapeParts * T;
         for (unsigned m = i; m < r.muscles; m += T) {
-            store(m).x = tape_at(k)[4u * T + m];
+            store(m).x = e[m];
         }
+    }
+    // What the rerun of substep k kept. Of the joint's gradients the hub's and
+    // the weight follow from the other two; the positions of a push are saved
+    // when there was one.
+    __device__ __forceinline__ void save_kept(unsigned k, const Kept& kept) const {
+        if (!has_node()) {
+            return;
+        }
+        const unsigned flags = (kept.pushed ? 1u : 0u) | (kept.touched ? 2u : 0u) | (kept.slid ? 4u : 0u);
+        part(k, kTapePulls) = pair(kept.pulls, kept.landing);
+        part(k, kTapeDrag) = pair(kept.drag0, kept.drag1);
+        part(k, kTapeBone) = pair(kept.bone0, kept.bone1);
+        part(k, kTapeHub) = make_float4(kept.vh.x, kept.vh.y, __uint_as_float(flags), 0.0f);
+        if (has_joint()) {
+            part(k, kTapeEnds) = pair(kept.vt, kept.vf);
+            part(k, kTapeTurn) = pair(kept.k.g_tip, kept.k.g_far);
+        }
+        if (kept.pushed) {
+            part(k, kTapeParent) = pair(kept.pt, kept.pp);
+            part(k, kTapeOwn) = pair(kept.ct, kept.ch);
+        }
+    }
+    struct Entry {
+        float4 state, pulls, drag, bone, ends, hub, turn;
+    };
+    __device__ __forceinline__ Entry entry_of(unsigned k) const {
+        const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        Entry e{none, none, none, none, none, none, none};
+        if (has_node()) {
+            e.state = part(k, kTapeState);
+            e.pulls = part(k, kTapePulls);
+            e.drag = part(k, kTapeDrag);
+            e.bone = part(k, kTapeBone);
+            e.hub = part(k, kTapeHub);
+            if (has_joint()) {
+                e.ends = part(k, kTapeEnds);
+                e.turn = part(k, kTapeTurn);
+            }
+        }
+        return e;
+    }
+    __device__ __forceinline__ Kept kept_of(unsigned k, const Entry& e) const {
+        const auto head = [](const float4& v) { return make_float2(v.x, v.y); };
+        const auto tail = [](const float4& v) { return make_float2(v.z, v.w); };
+        const unsigned flags = __float_as_uint(e.hub.z);
+        Kept kept;
+        kept.pulls = head(e.pulls);
+        kept.landing = tail(e.pulls);
+        kept.drag0 = head(e.drag);
+        kept.drag1 = tail(e.drag);
+        kept.bone0 = head(e.bone);
+        kept.bone1 = tail(e.bone);
+        kept.vt = head(e.ends);
+        kept.vf = tail(e.ends);
+        kept.vh = head(e.hub);
+        kept.pushed = (flags & 1u) != 0u;
+        kept.touched = (flags & 2u) != 0u;
+        kept.slid = (flags & 4u) != 0u;
+        kept.wgt = 0.0f;
+        if (has_joint()) {
+            kept.k.g_tip = head(e.turn);
+            kept.k.g_far = tail(e.turn);
+            P::complete(kept.k, rb);
+            kept.wgt = P::joint_weight(kept.k);
+        }
+        if (kept.pushed) {
+            const float4 parent = part(k, kTapeParent), own = part(k, kTapeOwn);
+            kept.pt = head(parent);
+            kept.pp = tail(parent);
+            kept.ct = head(own);
+            kept.ch = tail(own);
+        }
+        return kept;
     }
     __device__ __forceinline__ bool same(float x0, float x1) const { return __float_as_uint(x0) == __float_as_uint(x1); }
-    __device__ __forceinline__ bool same_as_tape(unsigned k) const {
-        bool ok = true;
-        if (has_node()) {
-            const float4 s = state_of(k);
-            const float2 q = pos(i), u = vel(i);
-            ok = same(s.x, q.x) && same(s.y, q.y) && same(s.z, u.x) && same(s.w, u.y);
-        }
-        for (unsigned m = i; m < r.muscles; m += T) {
-            ok = ok && same(tape_at(k)[4u * T + m], store(m).x);
-        }
-        return ok;
-    }
     __device__ __forceinline__ const float* checkpoint(unsigned s) const {
         return a.ckpt + (size_t)s * checkpoint_floats(a.rows, a.mm) * a.count + r.cidx;
     }
@@ -291,7 +360,9 @@ struct TeamBackward : Team<W, false, RATE, false> {
     }
 
     // The reverse of a substep (Backward::reverse_substep) from what its rerun
-    // kept and the state `s0` at its start (tape entry k_tape).
+    // kept and the state `s0` at its start (tape entry k_tape). Shared memory
+    // holds the positions at its end, the start of the one after, and then
+    // those at its start.
     __device__ __forceinline__ void reverse_substep(unsigned k_tape, const float4& s0, const Kept& kept) {
         const ce_params& p = f.p;
         const unsigned topo = __float_as_uint(ra.x);
@@ -530,8 +601,10 @@ struct TeamBackward : Team<W, false, RATE, false> {
             this->demands(__fmul_rn((float)(s0 + s), C::dt));
             __syncwarp();
             for (unsigned q = 0u; q < 16u; q++) {
+                Kept kept;
                 save_state(s * 16u + q);
-                this->substep();
+                this->template substep<true>(&kept);
+                save_kept(s * 16u + q, kept);
             }
             show(h);
             if (on && s + 1u == steps) {
@@ -554,23 +627,13 @@ struct TeamBackward : Team<W, false, RATE, false> {
             const Hidden h = hide(s >= steps);
             const float t_now = __fmul_rn((float)(s0 + s), C::dt);
             this->demands(t_now);
-            float4 state = state_of(s * 16u + 15u);
+            Entry now = entry_of(s * 16u + 15u);
             for (unsigned q = 16u; q-- > 0u;) {
                 const unsigned k = s * 16u + q;
-                put_state(k, state);
                 // The entry before comes while this substep is worked on.
-                const float4 next = q > 0u ? state_of(k - 1u) : state;
-                __syncwarp();
-                Kept kept;
-                this->template substep<true>(&kept);
-                if (x.mismatch && has_node()) {
-                    const bool last = k + 1u == steps * 16u;
-                    if (last ? (s0 + steps < end && !same_as_checkpoint(seg + 1u)) : !same_as_tape(k + 1u)) {
-                        atomicOr(x.mismatch + r.cidx, 2u);
-                    }
-                }
-                reverse_substep(k, state, kept);
-                state = next;
+                const Entry next = q > 0u ? entry_of(k - 1u) : now;
+                reverse_substep(k, now.state, kept_of(k, now));
+                now = next;
             }
             demands_back(t_now);
             show(h);

@@ -121,9 +121,6 @@ struct Physics {
         k.hub = topo & 31u;
         k.far = (topo >> 15u) & 31u;
         const bool at_head = ((topo >> 20u) & 1u) != 0u;
-        k.w_tip = rb.x;
-        k.w_far = rb.y;
-        k.w_hub = rb.z;
         const float2 u = make_float2(pt.x - pp.x, pt.y - pp.y);
         const float2 v = make_float2(ct.x - ch.x, ct.y - ch.y);
         const float uu = fmaxf(sum2(u.x, u.x, u.y, u.y), 1e-12f);
@@ -131,8 +128,15 @@ struct Physics {
         k.g_tip = make_float2(-v.y / vv, v.x / vv);
         const float2 g_u = make_float2(-u.y / uu, u.x / uu);
         k.g_far = at_head ? make_float2(-g_u.x, -g_u.y) : g_u;
-        k.g_hub = make_float2(-(k.g_tip.x + k.g_far.x), -(k.g_tip.y + k.g_far.y));
+        complete(k, rb);
         return k;
+    }
+    // The rest of a joint from the gradients of its tip and far nodes.
+    __device__ __forceinline__ static void complete(Joint& k, const float4& rb) {
+        k.w_tip = rb.x;
+        k.w_far = rb.y;
+        k.w_hub = rb.z;
+        k.g_hub = make_float2(-(k.g_tip.x + k.g_far.x), -(k.g_tip.y + k.g_far.y));
     }
     __device__ __forceinline__ static float joint_weight(const Joint& k) {
         const float tip = sum2(k.g_tip.x, k.g_tip.x, k.g_tip.y, k.g_tip.y);

@@ -599,7 +599,8 @@ ce_status ce_backward(ce_tape* tape, const float* dl_dfitness, float* grads, siz
 /* ce_backward that also checks its reruns against the forward run, to the
  * bit: per creature (packed order) `mismatches` gets bit 0 when a
  * segment's rerun from its checkpoint does not end on the next checkpoint
- * and bit 1 when a substep's kept rerun does not end on the next tape state;
+ * and bit 1 when a substep's kept rerun does not end on the next tape state
+ * (a batch on teams of lanes reruns a segment once, so it has no such rerun);
  * 0 everywhere means every gradient was taken along the forward run's own
  * trajectory. Slower than ce_backward (one more read of the state a
  * substep). */
