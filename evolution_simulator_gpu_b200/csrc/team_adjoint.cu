@@ -219,10 +219,6 @@ struct TeamBackward : Team<W, false, RATE, false> {
             s[m] = store(m).x;
         }
     }
-    // A substep's start state, as registers hold it until put_state().
-    __device__ __forceinline__ float4 state_of(unsigned k) const {
-        return has_node() ? part(k, kTapeState) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
     __device__ __forceinline__ void put_state(unsigned k, const float4& s) const {
         if (has_node()) {
             pos(i) = make_float2(s.x, s.y);
