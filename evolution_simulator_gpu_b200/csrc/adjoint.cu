@@ -524,11 +524,10 @@ struct Backward {
         // depth = radius - (q.y - height) / secant
         lq.y -= ldepth / sec;
         const float lheight = ldepth / sec;
-        float lsec = ldepth * (q.y - c.gr.x) / (sec * sec);
         // n = (-slope, 1) / secant, secant = sqrt(1 + slope^2)
-        float lslope = -lnx / sec;
-        lsec += (lnx * S - lny) / (sec * sec);
-        lslope += lsec * S / sec;
+        const float sec2 = sec * sec;
+        const float lsec = add_over((lnx * S - lny) / sec2, ldepth * (q.y - c.gr.x), sec2);
+        const float lslope = add_over(-lnx / sec, lsec * S, sec);
         lx += lheight * S + lslope * ground_curvature(b.w, q.x, b.r.amp, b.r.qphase);
         lq.x += lx;
         g.pos(i) = lq;
@@ -669,8 +668,8 @@ struct Backward {
             float ldx = w0 * sc * l0.x - w1 * sc * l1.x, ldy = w0 * sc * l0.y - w1 * sc * l1.y;
             if (len0 >= 1e-9f) {
                 const float llen = ls * ba.y / ((w0 + w1) * len * len);
-                ldx += llen * dx / len;
-                ldy += llen * dy / len;
+                ldx = add_over(ldx, llen * dx, len);
+                ldy = add_over(ldy, llen * dy, len);
             }
             g.pos(i0) = make_float2(l0.x - ldx, l0.y - ldy);
             g.pos(i1) = make_float2(l1.x + ldx, l1.y + ldy);
@@ -703,7 +702,7 @@ struct Backward {
                 const float y0 = tape.pair(k_tape, 2u * i)->y;
                 const float z = (p.water - (y0 - nr.z)) / (2.0f * nr.z);
                 if (z >= 0.0f && z <= 1.0f) {
-                    lp.y -= lv1.y * C::h * im * kWaterBuoyancy * nr.x * p.gravity / (2.0f * nr.z);
+                    lp.y = add_over(lp.y, -(lv1.y * C::h * im * kWaterBuoyancy * nr.x * p.gravity), 2.0f * nr.z);
                 }
             }
             g.pos(i) = lp;
@@ -774,20 +773,20 @@ struct Backward {
                 e.x -= lax / ba.y;
                 e.y -= lay / ba.y;
                 if (z0 >= 0.0f && z0 <= 1.0f) {
-                    e.y -= 0.5f * lwet / (2.0f * r0);
+                    e.y = add_over(e.y, -0.5f * lwet, 2.0f * r0);
                 }
                 g.pos(i0) = e;
                 e = g.pos(i1);
                 e.x += lax / ba.y;
                 e.y += lay / ba.y;
                 if (z1 >= 0.0f && z1 <= 1.0f) {
-                    e.y -= 0.5f * lwet / (2.0f * r1);
+                    e.y = add_over(e.y, -0.5f * lwet, 2.0f * r1);
                 }
                 g.pos(i1) = e;
             }
             if (speed > 0.0f) {
-                lwx += lspeed * wx / speed;
-                lwy += lspeed * wy / speed;
+                lwx = add_over(lwx, lspeed * wx, speed);
+                lwy = add_over(lwy, lspeed * wy, speed);
             }
             if (llimit != 0.0f) {
                 // The limit 0.5 (m0 + m1) / h.
@@ -1006,7 +1005,7 @@ struct Backward {
                     g_hill += lhc * lengthening;
                 }
             }
-            const float ld = ldrive0 * ms.x;
+            const float ld = __fmul_rn(ldrive0, ms.x);
             le += ldrive0 * ms.y;
             // Lengthening speed along the unit direction.
             const float lrvx = llg * ex, lrvy = llg * ey;
@@ -1014,10 +1013,10 @@ struct Backward {
             ley += llg * rvy;
             // e = d / len
             float ldx = lex / len, ldy = ley / len;
-            llen -= (lex * ex + ley * ey) / len;
+            llen = add_over(llen, -sum2(lex, ex, ley, ey), len);
             if (len0 >= 1e-6f) {
-                ldx += llen * dx / len;
-                ldy += llen * dy / len;
+                ldx = add_over(ldx, llen * dx, len);
+                ldy = add_over(ldy, llen * dy, len);
             }
             // Anchors on the two bones.
             float2 e;

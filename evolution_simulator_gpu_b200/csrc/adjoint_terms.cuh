@@ -39,14 +39,6 @@ __device__ __forceinline__ float ice_slope(float x) {
     return 6.0f * z * (1.0f - z) * -2.5f * dt;
 }
 
-// x + num / den as the compiler forms it of an approximate division: the
-// quotient's last product fused with the sum. (The empty statement keeps a
-// square root in `den` from turning the reciprocal into another one.)
-__device__ __forceinline__ float add_quotient(float x, float num, float den) {
-    asm("" : "+f"(den));
-    return __fmaf_rn(num, 1.0f / den, x);
-}
-
 // w -> perp(w) / |w|^2: its adjoint `lg` into w's (Backward::perp_back). The
 // damping's and the range test's copies fuse one sum each its own way.
 template <bool DAMPING>
@@ -180,8 +172,8 @@ __device__ __forceinline__ void bone_length_back(const float4& ba, const float4&
     float ldx = sum2(s0, l0.x, -s1, l1.x), ldy = sum2(s0, l0.y, -s1, l1.y);
     if (len0 >= 1e-9f) {
         const float llen = __fmul_rn(ls, ba.y) / __fmul_rn(__fmul_rn(__fadd_rn(w0, w1), len), len);
-        ldx = add_quotient(ldx, __fmul_rn(llen, dx), len);
-        ldy = add_quotient(ldy, __fmul_rn(llen, dy), len);
+        ldx = add_over(ldx, __fmul_rn(llen, dx), len);
+        ldy = add_over(ldy, __fmul_rn(llen, dy), len);
     }
     const float lsw = __fmul_rn(-ls, sc) / __fadd_rn(w0, w1);
     d0 = __fmaf_rn(sc, sum2(dx, l0.x, dy, l0.y), lsw);
@@ -208,7 +200,7 @@ __device__ __forceinline__ void integrate_back(const W& w, const ce_params& p, c
         if (z >= 0.0f && z <= 1.0f) {
             const float lift = __fmul_rn(
                 __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(lv1.y, C::h), im), kWaterBuoyancy), nr.x), p.gravity);
-            lp.y = add_quotient(lp.y, -lift, 2.0f * nr.z);
+            lp.y = add_over(lp.y, -lift, 2.0f * nr.z);
         }
     }
     lf = make_float2(__fmul_rn(__fmul_rn(lv1.x, C::h), im), __fmul_rn(__fmul_rn(lv1.y, C::h), im));
@@ -272,12 +264,12 @@ __device__ __forceinline__ void bone_drag_back(const W& w, const ce_params& p, c
         e0.x = __fadd_rn(e0.x, -lax / ba.y);
         e0.y = __fadd_rn(e0.y, -lay / ba.y);
         if (z0 >= 0.0f && z0 <= 1.0f) {
-            e0.y = add_quotient(e0.y, -0.5f * lwet, 2.0f * r0);
+            e0.y = add_over(e0.y, -0.5f * lwet, 2.0f * r0);
         }
         e1.x = __fadd_rn(e1.x, lax / ba.y);
         e1.y = __fadd_rn(e1.y, lay / ba.y);
         if (z1 >= 0.0f && z1 <= 1.0f) {
-            e1.y = add_quotient(e1.y, -0.5f * lwet, 2.0f * r1);
+            e1.y = add_over(e1.y, -0.5f * lwet, 2.0f * r1);
         }
     } else {
         lwx = __fmul_rn(-k_air, ldx);
@@ -286,8 +278,8 @@ __device__ __forceinline__ void bone_drag_back(const W& w, const ce_params& p, c
         dfy = __fmul_rn(-wy, k_air);
     }
     if (speed > 0.0f) {
-        lwx = add_quotient(lwx, __fmul_rn(lspeed, wx), speed);
-        lwy = add_quotient(lwy, __fmul_rn(lspeed, wy), speed);
+        lwx = add_over(lwx, __fmul_rn(lspeed, wx), speed);
+        lwy = add_over(lwy, __fmul_rn(lspeed, wy), speed);
     }
     d0 = __fmul_rn(0.5f * C::h, sum2(l0.x, dfx, l0.y, dfy));
     d1 = __fmul_rn(0.5f * C::h, sum2(l1.x, dfx, l1.y, dfy));
@@ -346,8 +338,8 @@ __device__ __forceinline__ void contact_back(const W& w, const ce_params& p, flo
     lq.y = __fadd_rn(lq.y, -ldepth / sec);
     const float lheight = ldepth / sec;
     const float sec2 = __fmul_rn(sec, sec);
-    const float lsec = add_quotient(__fmaf_rn(lnx, S, -lny) / sec2, __fmul_rn(ldepth, q.y - gr.x), sec2);
-    const float lslope = add_quotient(-lnx / sec, __fmul_rn(lsec, S), sec);
+    const float lsec = add_over(__fmaf_rn(lnx, S, -lny) / sec2, __fmul_rn(ldepth, q.y - gr.x), sec2);
+    const float lslope = add_over(-lnx / sec, __fmul_rn(lsec, S), sec);
     lx += sum2(lheight, S, lslope, ground_curvature(w, q.x, amp, qphase));
     lq.x += lx;
     lq_io = lq;
@@ -432,10 +424,10 @@ __device__ __forceinline__ void muscle_back(const ce_params& p, const float4& q0
     out.lrvy = __fmul_rn(llg, ey);
     const float lex = sum2(llg, rvx, lfx, pull), ley = sum2(llg, rvy, lfy, pull);
     float ldx = lex / len, ldy = ley / len;
-    llen = add_quotient(llen, -sum2(lex, ex, ley, ey), len);
+    llen = add_over(llen, -sum2(lex, ex, ley, ey), len);
     if (len0 >= 1e-6f) {
-        ldx = add_quotient(ldx, __fmul_rn(llen, dx), len);
-        ldy = add_quotient(ldy, __fmul_rn(llen, dy), len);
+        ldx = add_over(ldx, __fmul_rn(llen, dx), len);
+        ldy = add_over(ldy, __fmul_rn(llen, dy), len);
     }
     out.ldx = ldx;
     out.ldy = ldy;

@@ -53,6 +53,21 @@ constexpr float kPiF = 3.14159265359f;
 constexpr float kTauF = 6.28318530718f;
 constexpr uint32_t kNone = 0xffffffffu;
 
+// a b + c d with the first product fused.
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) {
+    return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+
+// 1 / x by PTX's approximate reciprocal (to one unit in the last place).
+__device__ __forceinline__ float inverse(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// x + num / den as one multiply-add with the denominator's reciprocal: the
+// two backward kernels (adjoint.cu, team_adjoint.cu) form these sums alike.
+__device__ __forceinline__ float add_over(float x, float num, float den) { return __fmaf_rn(num, inverse(den), x); }
+
 // Step clock of a fidelity: RATE steps per second, 16 substeps per step.
 template <int RATE>
 struct Clock {

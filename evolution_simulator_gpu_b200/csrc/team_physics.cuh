@@ -15,11 +15,6 @@
 
 namespace cek {
 
-// a b + c d with the first product fused.
-__device__ __forceinline__ float sum2(float a, float b, float c, float d) {
-    return __fmaf_rn(a, b, __fmul_rn(c, d));
-}
-
 // Ground height and slope under x (shaders/creature.cu:166-226).
 // `BACK`: as the backward run's contact fuses it.
 template <bool BACK = false, class W>
