@@ -153,7 +153,8 @@ class GenSpec(C.Structure):
 
 class Options(C.Structure):
     _fields_ = [("slots", C.c_uint32), ("ctas_per_sm", C.c_uint32), ("warps_per_cta", C.c_uint32),
-                ("chunk_k", C.c_uint32), ("small_body", C.c_uint32), ("reserved", C.c_uint32 * 3)]
+                ("chunk_k", C.c_uint32), ("small_body", C.c_uint32), ("teams", C.c_uint32),
+                ("reserved", C.c_uint32 * 2)]
 
 
 # --------------------------------------------------------------- library
@@ -557,12 +558,15 @@ class Engine:
     """One GPU's engine (the reference's ThreadedEngine surface)."""
 
     def __init__(self, device: int = 0, slots: int = 0, ctas_per_sm: int = 0, chunk_k: int = 0,
-                 small_body: int = 0):
+                 small_body: int = 0, teams: int = 0):
         """`ctas_per_sm` (0: as many as fit), `chunk_k` (creatures a warp
         claims per queue visit, 0: 64) and `small_body` (largest node count run
-        as a small body, 0: 12) are the launch shape; `autotune` picks them."""
+        as a small body, 0: 12) are the shape of launches of one creature a
+        lane; `autotune` picks them. `teams`: small launches and the last
+        trials of large ones on teams of lanes where that is the faster (1) or
+        never (2); 0 is 1 unless `ctas_per_sm` is given."""
         h = C.c_void_p()
-        opts = Options(slots, ctas_per_sm, 0, chunk_k, small_body)
+        opts = Options(slots, ctas_per_sm, 0, chunk_k, small_body, teams)
         _check(lib().ce_open(device, C.byref(opts), C.byref(h)), "ce_open")
         self._h = h
         self.device = device
@@ -570,12 +574,14 @@ class Engine:
     def autotune(self, sample: WavePack, world: World) -> tuple[dict, float]:
         """Time `sample` under each launch shape (CTAs per SM x claim chunk x
         small-body bound) and keep the fastest for later submissions:
-        ({ctas_per_sm, chunk_k, small_body}, its GPU-busy seconds). Results do
-        not depend on the launch shape."""
+        ({ctas_per_sm, chunk_k, small_body, teams}, its GPU-busy seconds); an
+        engine opened with these runs as this one. Results do not depend on
+        the launch shape."""
         best, secs = Options(), C.c_double()
         _check(lib().ce_autotune(self.handle, C.byref(sample.c()), C.byref(world), C.byref(best), C.byref(secs)),
                "ce_autotune")
-        return {"ctas_per_sm": best.ctas_per_sm, "chunk_k": best.chunk_k, "small_body": best.small_body}, secs.value
+        return {"ctas_per_sm": best.ctas_per_sm, "chunk_k": best.chunk_k, "small_body": best.small_body,
+                "teams": best.teams}, secs.value
 
     @property
     def handle(self) -> C.c_void_p:

@@ -111,6 +111,8 @@ struct ce_engine {
     int device = 0;
     int sms = 0;
     unsigned ctas_per_sm = 0;  // 0: from the occupancy of each kernel
+    bool teams = true;         // small launches and the last trials of large ones on teams of lanes
+    bool tuning = false;       // ce_autotune times a sample: every creature starts on a lane
     unsigned chunk_k = 64;
     size_t smem_optin = 0;  // shared memory a block may use
     size_t smem_sm = 0;     // shared memory of an SM
@@ -195,18 +197,17 @@ std::vector<unsigned> class_grids(ce_engine* e, const std::vector<ClassPlan>& pl
 // meet between 16,000 creatures of 3 to 6 nodes and 200,000 of 3 to 24 nodes
 // in the effects world (5 s trials, ms on teams / on lanes: small 16,384
 // 27.7 / 31.0 and 32,768 43.8 / 41.5; game 32,768 71 / 92 and 65,536 130 /
-// 108; effects 131,072 149 / 211 and 262,144 283 / 233). A caller that sets
-// the blocks an SM asks for the lane kernel's launch shape and gets it.
+// 108; effects 131,072 149 / 211 and 262,144 283 / 233).
 constexpr size_t kTeamMost = 24576;
 constexpr unsigned kTailMost = 24576;
-bool team_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamMost; }
+bool team_pays(const ce_engine* e, size_t count) { return e->teams && !e->tuning && count <= kTeamMost; }
 
 // Whether a backward run of `count` creatures goes on teams: the same trade
 // (ms on teams / on lanes: calm x 2 s 8,192 59 / 176, 16,384 107 / 188, 32,768
 // 195 / 206, 49,152 287 / 241; the refined search's world x 4 s 16,384 176 /
 // 473, 32,768 313 / 536, 65,536 594 / 725).
 constexpr size_t kTeamBackMost = 32768;
-bool team_back_pays(const ce_engine* e, size_t count) { return e->ctas_per_sm == 0 && count <= kTeamBackMost; }
+bool team_back_pays(const ce_engine* e, size_t count) { return e->teams && count <= kTeamBackMost; }
 
 ce_status check_world(const ce_world* w) {
     if (!w) {
@@ -308,7 +309,7 @@ struct LaunchPlan {
 
 // Creatures left at which a lane launch hands its trials over to teams.
 unsigned tail_most(const ce_engine* e, size_t count) {
-    return e->ctas_per_sm == 0 && count > kTeamMost ? kTailMost : 0u;
+    return e->teams && count > kTeamMost ? kTailMost : 0u;
 }
 
 ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, int rate, LaunchPlan& lp) {
@@ -437,6 +438,7 @@ extern "C" ce_status ce_open(int device, const ce_options* options, ce_engine** 
     if (options) {
         if (options->slots) nslots = options->slots;
         e->ctas_per_sm = options->ctas_per_sm;
+        e->teams = options->teams == 1u || (options->teams != 2u && options->ctas_per_sm == 0);
         if (options->chunk_k) e->chunk_k = options->chunk_k;
         if (options->small_body) e->small_body = std::min<unsigned>(options->small_body, CE_MAX_NODES);
     }
@@ -750,7 +752,7 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
 }
 
 // The device entry's scratch: the lane slots of the grid, then the claim
-// queues of `count` creatures.
+// queues of `count` creatures, then the tail.
 namespace {
 size_t slots_part(ce_engine* e, uint32_t world_flags, uint32_t rate, uint32_t max_nodes, uint32_t max_muscles) {
     const unsigned grid = grid_for(e, max_nodes, max_muscles, world_flags, false, (int)rate, (size_t)1 << 30);
@@ -1697,6 +1699,13 @@ extern "C" ce_status ce_autotune(ce_engine* e, const ce_wave_pack* sample, const
     }
     const unsigned keep_cta = e->ctas_per_sm, keep_chunk = e->chunk_k, keep_small = e->small_body;
     std::vector<ce_result> out(sample->count);
+    // A sample that would run on teams tells nothing of the settings, which
+    // shape the lane kernel's launches: here every creature starts on a lane.
+    struct Tuning {
+        ce_engine* e;
+        explicit Tuning(ce_engine* engine) : e(engine) { e->tuning = true; }
+        ~Tuning() { e->tuning = false; }
+    } const tuning(e);
     auto time_one = [&](double* busy) -> ce_status {
         uint64_t ticket = 0, got = 0;
         ce_status s = ce_submit(e, sample, w, &ticket);
@@ -1740,6 +1749,7 @@ extern "C" ce_status ce_autotune(ce_engine* e, const ce_wave_pack* sample, const
         best->ctas_per_sm = best_cta;
         best->chunk_k = best_chunk;
         best->small_body = best_small;
+        best->teams = e->teams ? 1u : 2u;
     }
     if (seconds) *seconds = best_s;
     return CE_OK;
