@@ -111,6 +111,7 @@ struct ce_engine {
     int device = 0;
     int sms = 0;
     unsigned ctas_per_sm = 0;  // 0: from the occupancy of each kernel
+    unsigned opened_ctas = 0;  // as opened; ce_autotune changes ctas_per_sm
     bool teams = true;         // small launches and the last trials of large ones on teams of lanes
     bool tuning = false;       // ce_autotune times a sample: every creature starts on a lane
     unsigned chunk_k = 64;
@@ -131,11 +132,13 @@ namespace {
 
 ce_status set_device(ce_engine* e) { return cuda_status(cudaSetDevice(e->device), "cudaSetDevice"); }
 
-// The grid of a persistent launch for a class: every block that fits.
-unsigned grid_for(ce_engine* e, unsigned rows, unsigned mm, uint32_t flags, bool record, int rate, size_t count) {
+// The grid of a persistent launch for a class, of `ctas` blocks an SM (0:
+// every block that fits).
+unsigned grid_of(ce_engine* e, unsigned ctas, unsigned rows, unsigned mm, uint32_t flags, bool record, int rate,
+                 size_t count) {
     int per_sm = 0;
-    if (e->ctas_per_sm) {
-        per_sm = (int)e->ctas_per_sm;
+    if (ctas) {
+        per_sm = (int)ctas;
     } else if (cek::advance_occupancy(rows, mm, flags, record, rate, cek::kBlock, &per_sm) != cudaSuccess ||
                per_sm < 1) {
         cudaGetLastError();
@@ -144,6 +147,10 @@ unsigned grid_for(ce_engine* e, unsigned rows, unsigned mm, uint32_t flags, bool
     const size_t needed = (count + cek::kBlock - 1) / cek::kBlock;
     const size_t full = (size_t)per_sm * (size_t)e->sms;
     return (unsigned)std::max<size_t>(1, std::min(needed, full));
+}
+
+unsigned grid_for(ce_engine* e, unsigned rows, unsigned mm, uint32_t flags, bool record, int rate, size_t count) {
+    return grid_of(e, e->ctas_per_sm, rows, mm, flags, record, rate, count);
 }
 
 size_t scratch_bytes(unsigned grid, unsigned rows, unsigned mm, bool record) {
@@ -437,7 +444,7 @@ extern "C" ce_status ce_open(int device, const ce_options* options, ce_engine** 
     unsigned nslots = 4;
     if (options) {
         if (options->slots) nslots = options->slots;
-        e->ctas_per_sm = options->ctas_per_sm;
+        e->ctas_per_sm = e->opened_ctas = options->ctas_per_sm;
         e->teams = options->teams == 1u || (options->teams != 2u && options->ctas_per_sm == 0);
         if (options->chunk_k) e->chunk_k = options->chunk_k;
         if (options->small_body) e->small_body = std::min<unsigned>(options->small_body, CE_MAX_NODES);
@@ -752,10 +759,18 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
 }
 
 // The device entry's scratch: the lane slots of the grid, then the claim
-// queues of `count` creatures, then the tail.
+// queues of `count` creatures, then the tail. A caller sizes it once, and
+// ce_autotune may change the blocks an SM after that, so the slots are those
+// of the largest grid that the handle can come to launch.
 namespace {
+constexpr unsigned kTunedCtas[2] = {0u, 3u};
 size_t slots_part(ce_engine* e, uint32_t world_flags, uint32_t rate, uint32_t max_nodes, uint32_t max_muscles) {
-    const unsigned grid = grid_for(e, max_nodes, max_muscles, world_flags, false, (int)rate, (size_t)1 << 30);
+    unsigned grid = 0;
+    const auto take = [&](unsigned ctas) {
+        grid = std::max(grid, grid_of(e, ctas, max_nodes, max_muscles, world_flags, false, (int)rate, (size_t)1 << 30));
+    };
+    for (const unsigned ctas : kTunedCtas) take(ctas);
+    if (e->opened_ctas) take(e->opened_ctas);
     return (scratch_bytes(grid, max_nodes, max_muscles, false) + 255u) & ~(size_t)255u;
 }
 }  // namespace
@@ -1718,7 +1733,7 @@ extern "C" ce_status ce_autotune(ce_engine* e, const ce_wave_pack* sample, const
     if (s != CE_OK) return s;
     double best_s = 1e300;
     unsigned best_cta = keep_cta, best_chunk = keep_chunk, best_small = keep_small;
-    for (unsigned cta : {0u, 3u}) {
+    for (unsigned cta : kTunedCtas) {
         for (unsigned chunk : {16u, 32u, 64u}) {
             for (unsigned small : {10u, 12u, 16u, 24u}) {
                 e->ctas_per_sm = cta;

@@ -493,7 +493,8 @@ ce_status ce_open(int device, const ce_options* options, ce_engine** out);
  * grid of launch settings of one creature a lane (blocks an SM, claim chunk
  * divisor, size-class split) and keeps the fastest for the engine's later
  * submissions; `best` (optional) receives it and `seconds` (optional) its GPU
- * time. Which launches go on teams stays as opened. No counterpart in the
+ * time. Which launches go on teams stays as opened, and scratch sized by
+ * ce_advance_scratch_bytes before stays large enough. No counterpart in the
  * reference, whose launch shape is fixed. */
 ce_status ce_autotune(ce_engine* engine, const ce_wave_pack* sample, const ce_world* world, ce_options* best,
                       double* seconds);

@@ -45,3 +45,19 @@ def test_teams_are_chosen_when_an_engine_is_opened(opts, teams):
         best, _ = e.autotune(small, world)
         assert best["teams"] == (1 if teams else 2)
         assert all((a > b) == teams for a, b in zip(large, scratch(lanes, world, 300_000)))
+
+
+@pytest.mark.parametrize("count", [1, 1000, 300_000])
+def test_scratch_does_not_depend_on_what_the_tuner_changes(count):
+    """The autotuner sets 0 or 3 blocks an SM on any engine: scratch sized
+    before has to hold the largest grid it may choose. Nothing is launched
+    into the scratch here."""
+    world = ce.make_world(duration=1.0)
+    small = ce.pack(ce.generate(WORKLOADS["small"].spec, 300), world)
+    with ce.Engine(0) as plain:
+        want = scratch(plain, world, count)
+    for ctas in (1, 2, 3):
+        with ce.Engine(0, ctas_per_sm=ctas, teams=1) as e:
+            assert scratch(e, world, count) == want
+            e.autotune(small, world)
+            assert scratch(e, world, count) == want
