@@ -1182,7 +1182,7 @@ __global__ void __launch_bounds__(kBlock, 2) adjoint_kernel(const KernelArgs a, 
     bool live = false;
     Claim claim(a, lane, warp, warps_total);
     for (;;) {
-        const unsigned mine = claim.next(live || lane >= a.lanes);
+        const unsigned mine = claim.next(live);
         unsigned done_cidx = kNone;
         if (mine != kNone) {
             const unsigned cidx = a.order ? __ldg(a.order + mine) : p.base + mine;
@@ -1207,23 +1207,6 @@ __global__ void __launch_bounds__(kBlock, 2) adjoint_kernel(const KernelArgs a, 
 }
 
 }  // namespace
-
-// A warp works as long as the longest of its lanes' trials needs and pays
-// for each side of every branch that some lane takes, so a batch that leaves
-// schedulers without a warp spreads over all of them, a few lanes in each:
-// 1,021 creatures x 10 s of the refined search's world 1,024 -> 657 ms. With a
-// warp on every scheduler full warps are better (16,381 calm creatures x 4 s:
-// 360 ms, and 375 ms as two half-filled warps a scheduler). Batches as small
-// as that run here where the caller set the blocks an SM; others go on teams.
-AdjointGrid adjoint_grid(size_t count, size_t sms, size_t blocks) {
-    constexpr size_t per = kBlock / 32u;
-    const size_t lanes = (count + sms * per - 1u) / (sms * per);
-    AdjointGrid g;
-    g.lanes = (unsigned)(lanes < 1u ? 1u : lanes > 32u ? 32u : lanes);
-    const size_t need = (count + g.lanes * per - 1u) / (g.lanes * per);
-    g.grid = (unsigned)(need < 1u ? 1u : need < blocks ? need : blocks);
-    return g;
-}
 
 size_t adjoint_smem_bytes(unsigned rows, unsigned mm, unsigned block) {
     return (size_t)block * (rows * 44u + (mm > 0u ? mm : 1u) * 16u);

@@ -1063,8 +1063,8 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
         cudaGetLastError();
         per_sm = 1;
     }
-    const cek::AdjointGrid ag = cek::adjoint_grid(t->count, (size_t)t->engine->sms, (size_t)per_sm * t->engine->sms);
-    const unsigned grid = ag.grid;
+    const size_t needed = (t->count + cek::kBlock - 1) / cek::kBlock;
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min(needed, (size_t)per_sm * t->engine->sms));
     const bool team = team_back_pays(t->engine, t->count);
     unsigned blocks = 0;
     if (team) {
@@ -1092,7 +1092,6 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
     CE_TRY(cek::launch_bucket(static_cast<const uint4*>(t->d_heads.ptr), 0u, (uint32_t)t->count, bk, st),
            "bucketing launch");
     cek::KernelArgs a = tape_args(t, bk);
-    a.lanes = ag.lanes;
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
     const float* weights = dl_dfitness ? static_cast<const float*>(t->d_weights.ptr) : nullptr;
     uint32_t* mismatch = mismatches ? static_cast<uint32_t*>(t->d_mismatch.ptr) : nullptr;
@@ -1364,8 +1363,8 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         cudaGetLastError();
         per_sm = 1;
     }
-    const cek::AdjointGrid ag = cek::adjoint_grid(n, (size_t)e->sms, (size_t)per_sm * e->sms);
-    const unsigned bgrid = ag.grid;
+    const unsigned bgrid =
+        (unsigned)std::max<size_t>(1, std::min((n + cek::kBlock - 1) / cek::kBlock, (size_t)per_sm * e->sms));
     const bool team_back = team_back_pays(e, n);
     unsigned bblocks = 0;
     if (team_back && (s = cuda_status(cek::team_adjoint_blocks(a->rows, a->mm, flags, a->rate, (unsigned)e->sms, n, &bblocks),
@@ -1423,7 +1422,6 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         k.rows = a->rows;
         k.mm = a->mm;
         k.chunk_k = e->chunk_k;
-        k.lanes = ag.lanes;
         k.ckpt = static_cast<float*>(a->d_ckpt.ptr);
         k.ends = static_cast<uint32_t*>(a->d_ends.ptr);
         return k;

@@ -77,7 +77,6 @@ struct KernelArgs {
     uint32_t mm;                   // most muscles of a body of this launch
     uint32_t frames_per_creature;  // RECORD: frames of one recording
     uint32_t chunk_k;              // claims shrink to 1 / chunk_k of the rest per warp
-    uint32_t lanes;                // lanes of a warp that take creatures (backward run; 32 elsewhere)
     float* ckpt;                   // CKPT: checkpoints, creature-minor: float f of checkpoint k of
                                    // creature c (packed index) at (k * checkpoint_floats + f) * count + c
     uint32_t* ends;                // CKPT: steps each creature's trial ran (packed index)
@@ -115,12 +114,6 @@ size_t adjoint_slot_bytes(unsigned grid, unsigned rows, unsigned mm);   // lane 
 size_t adjoint_tape_bytes(unsigned grid, unsigned rows, unsigned mm);   // segment tapes of the backward grid
 // Worlds the gradient kernels are built for: calm, effects, effects + tremors.
 bool gradient_world(uint32_t flags);
-// Lanes of a warp that take creatures, and the grid, of a backward run of
-// `count` creatures on `sms` multiprocessors that hold `blocks` blocks.
-struct AdjointGrid {
-    unsigned grid, lanes;
-};
-AdjointGrid adjoint_grid(size_t count, size_t sms, size_t blocks);
 cudaError_t adjoint_occupancy(unsigned rows, unsigned mm, uint32_t flags, int rate, int* blocks);
 struct LaunchSpec;
 cudaError_t launch_forward_ckpt(const LaunchSpec& s, const KernelArgs& a, const ce_params& p);
