@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <deque>
@@ -92,6 +93,7 @@ struct ClassPlan {
     uint32_t rows;             // most nodes in the class
     uint32_t mm;               // most muscles in the class
     double work;               // estimated arithmetic of a substep of all its creatures
+    double load;               // a substep of all its creatures on teams (team_load), ns
 };
 
 struct Slot {
@@ -197,24 +199,79 @@ std::vector<unsigned> class_grids(ce_engine* e, const std::vector<ClassPlan>& pl
     return grids;
 }
 
-// Whether `count` creatures run on teams of lanes (team.cuh) instead of one
-// creature a lane. A launch of few creatures takes as long as its longest
-// trial, which teams shorten 2 to 7 times; a launch of many is bound by
-// instruction issue, of which a team spends about 2.4 times a lane's. The two
-// meet between 16,000 creatures of 3 to 6 nodes and 200,000 of 3 to 24 nodes
-// in the effects world (5 s trials, ms on teams / on lanes: small 16,384
-// 27.7 / 31.0 and 32,768 43.8 / 41.5; game 32,768 71 / 92 and 65,536 130 /
-// 108; effects 131,072 149 / 211 and 262,144 283 / 233).
+// Teams of lanes (team.cuh) or one creature a lane: a launch of few creatures
+// takes on lanes as long as its longest trial, one substep after the other;
+// on teams as long as their warps' issue takes on all schedulers, the sum
+// over the creatures. Both are linear in the body's size. Measured on 148 SMs
+// in the calm world, bodies of one size, ns a substep (trials of 0.3 s, in
+// which few creatures fall; on lanes 12,288 of them, on teams 24,576, a
+// creature; in brackets the model below, whose teams cost a tenth more for
+// the part-filled last wave of fewer creatures):
+//
+//     nodes, muscles      3, 1   6, 8   8, 24   9, 1   12, 24   17, 8   32, 96
+//     on lanes            2,750  6,920  16,070  7,820  20,580   22,020  65,870
+//     lane_chain         (1,850  6,600  15,000  7,500  19,800   21,300  64,000)
+//     on teams             0.28   0.45    0.60   0.86    1.10     2.08    2.94
+//     team_cost           (0.34   0.49    0.70   0.96    1.19     2.22    3.26)
+//
+// So 5,500 bodies of 3 nodes or 9,600 of 17 take as long either way, and
+// 21,000 of 8 nodes. Creatures that fall leave their teams to others but do
+// not shorten the longest trial: with many falls teams are ahead of this.
+// Up to which count teams were measured:
 constexpr size_t kTeamMost = 24576;
-constexpr unsigned kTailMost = 24576;
-bool team_pays(const ce_engine* e, size_t count) { return e->teams && !e->tuning && count <= kTeamMost; }
-
-// Whether a backward run of `count` creatures goes on teams: the same trade
-// (ms on teams / on lanes: calm x 2 s 8,192 59 / 176, 16,384 107 / 188, 32,768
-// 195 / 206, 49,152 287 / 241; the refined search's world x 4 s 16,384 176 /
-// 473, 32,768 313 / 536, 65,536 594 / 725).
 constexpr size_t kTeamBackMost = 32768;
-bool team_back_pays(const ce_engine* e, size_t count) { return e->teams && count <= kTeamBackMost; }
+
+// A substep of one creature on a lane.
+double lane_chain(unsigned nodes, unsigned muscles) {
+    // Blocks with small tables leave more of the SM's memory to the L1 cache.
+    const double cached = 24u * nodes + 8u * muscles < 240u ? 250.0 * nodes : 0.0;
+    return std::max(1200.0 * nodes + 280.0 * muscles - 1300.0 - cached, 500.0 * nodes);
+}
+// A creature's share of a substep of all schedulers on teams: its team's
+// lanes take turns at the muscles.
+double team_cost(unsigned nodes, unsigned muscles) {
+    const unsigned lanes = nodes <= 8u ? 8u : nodes <= 16u ? 16u : 32u;
+    const double base = lanes == 8u ? 0.13 + 0.05 * nodes : (lanes == 16u ? 0.5 : 1.34) + 0.0385 * nodes;
+    const unsigned turns = std::max(1u, (muscles + lanes - 1u) / lanes);
+    return base + 0.0072 * lanes * turns;
+}
+// Where the creatures' shared memory leaves room for fewer blocks an SM than
+// 8, latency shows (96 muscles on 8 lanes: 3 blocks, 1.44 ns instead of 0.9).
+// `first_n`: fewest nodes of a body, of whose team's size the memory is too.
+double team_load(const ce_engine* e, double costs, unsigned first_n, unsigned rows, unsigned mm) {
+    const double fit = (double)(e->smem_sm / (cek::team_smem_bytes(first_n, rows, mm) + e->smem_reserved));
+    return costs * std::sqrt(cek::kTeamMinBlocks / std::clamp(fit, 1.0, (double)cek::kTeamMinBlocks)) *
+           (148.0 / e->sms);
+}
+// Whether a launch of `load` (ns a substep) goes on teams. More creatures than
+// the lanes hold at once (96 muscles: 18,944) take the lanes another round (ms
+// a 0.3 s trial of 8 nodes and 96 muscles on lanes / on teams: 18,432
+// creatures 10.9 / 8.7, 24,576 20.8 / 11.6).
+bool team_pays(ce_engine* e, size_t count, double load, unsigned rows, unsigned mm, uint32_t flags, bool record,
+               int rate) {
+    if (!e->teams || e->tuning || count > kTeamMost) return false;
+    const double chain = lane_chain(rows, mm);
+    if (load <= chain) return true;
+    const size_t lanes = (size_t)grid_for(e, rows, mm, flags, record, rate, (size_t)1 << 30) * cek::kBlock;
+    return load <= chain * (double)((count + lanes - 1) / lanes);
+}
+// Creatures left at which a lane launch of `load` hands its trials over to
+// teams: three quarters of those that teams pay for beside `others` (ns a
+// substep) on teams already, each taken for an average one; 0 for none.
+unsigned tail_most(const ce_engine* e, size_t count, double load, double others, unsigned rows, unsigned mm) {
+    if (!e->teams || e->tuning || count == 0) return 0u;
+    const double most = std::min(0.75 * lane_chain(rows, mm) * (double)count / (load + others), (double)kTeamMost);
+    return (double)count > most ? (unsigned)most : 0u;
+}
+// Whether a backward run goes on teams: the same trade, 6 times the forward
+// load against 5 times its chain, and again for each round of `lanes` (ms a
+// 1 s trial on teams / on lanes, calm: 8,192 bodies of 3 nodes 13.6 / 11.2, 9
+// nodes 40 / 45, 17 nodes 90 / 95; 16,384 of 8 nodes 42 / 50, 12 nodes 91 /
+// 85, 17 nodes 173 / 107; 32,768 of 8 nodes and 48 muscles 136 / 226).
+bool team_back_pays(const ce_engine* e, size_t count, double load, unsigned rows, unsigned mm, size_t lanes) {
+    if (!e->teams || count > kTeamBackMost) return false;
+    return 6.0 * load <= 5.0 * lane_chain(rows, mm) * (double)((count + lanes - 1) / lanes);
+}
 
 ce_status check_world(const ce_world* w) {
     if (!w) {
@@ -273,7 +330,7 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
     plans.clear();
     size_t per_n[CE_MAX_NODES + 1] = {};
     uint32_t mm_n[CE_MAX_NODES + 1] = {};
-    double work_n[CE_MAX_NODES + 1] = {};
+    double work_n[CE_MAX_NODES + 1] = {}, cost_n[CE_MAX_NODES + 1] = {};
     for (size_t i = 0; i < pack->count; i++) {
         const uint32_t* h = pack->heads + 8 * i;
         const unsigned n = h[0] & 255u, m = h[1];
@@ -286,9 +343,10 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
         mm_n[n] = std::max(mm_n[n], m);
         // Operations of a substep: 75 a muscle, 40 a bone, 36 a node, 110 a joint.
         work_n[n] += 75.0 * m + 40.0 * (n - 1) + 36.0 * n + 110.0 * (n >= 2 ? n - 2 : 0);
+        cost_n[n] += team_cost(n, m);
     }
     for (int big = 0; big < 2; big++) {
-        ClassPlan c{0, 0, 0, 2, 0, 0.0};
+        ClassPlan c{0, 0, 0, 2, 0, 0.0, 0.0};
         for (unsigned n = 2; n <= CE_MAX_NODES; n++) {
             if (per_n[n] == 0 || (n > small_body) != (big != 0)) continue;
             if (c.count == 0) c.first_n = n;
@@ -297,6 +355,7 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
             c.rows = n;
             c.mm = std::max(c.mm, mm_n[n]);
             c.work += work_n[n];
+            c.load += cost_n[n];
         }
         if (c.count) plans.push_back(c);
     }
@@ -310,41 +369,52 @@ struct LaunchPlan {
     std::vector<char> team;
     std::vector<unsigned> grids;             // of the lane launches
     std::vector<size_t> slots_at, tail_at;   // offsets in the scratch
+    std::vector<unsigned> tail;              // creatures that each lane launch hands over
     size_t scratch = 0;
-    unsigned tail = 0;
 };
 
-// Creatures left at which a lane launch hands its trials over to teams.
-unsigned tail_most(const ce_engine* e, size_t count) {
-    return e->teams && count > kTeamMost ? kTailMost : 0u;
+// All classes as one, for what serves every node count in one launch.
+ClassPlan whole(const std::vector<ClassPlan>& plans) {
+    ClassPlan all = plans[0];
+    for (size_t c = 1; c < plans.size(); c++) {
+        all.last_n = plans[c].last_n;
+        all.rows = std::max(all.rows, plans[c].rows);
+        all.mm = std::max(all.mm, plans[c].mm);
+        all.count += plans[c].count;
+        all.load += plans[c].load;
+    }
+    return all;
 }
 
 ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, int rate, LaunchPlan& lp) {
     lp = LaunchPlan{};
     ce_status s = plan_classes(pack, lp.classes, e->small_body);
     if (s != CE_OK || lp.classes.empty()) return s;
-    if (team_pays(e, pack->count)) {
-        // One launch serves every node count.
-        ClassPlan all = lp.classes[0];
-        for (const ClassPlan& c : lp.classes) {
-            all.last_n = c.last_n;
-            all.rows = std::max(all.rows, c.rows);
-            all.mm = std::max(all.mm, c.mm);
-        }
-        all.count = (uint32_t)pack->count;
-        lp.classes.assign(1, all);
-    }
+    const auto pays = [&](const ClassPlan& c, double load) {
+        return team_pays(e, c.count, load, c.rows, c.mm, flags, false, rate);
+    };
+    const ClassPlan all = whole(lp.classes);
+    if (pays(all, team_load(e, all.load, all.first_n, all.rows, all.mm))) lp.classes.assign(1, all);
     const size_t n = lp.classes.size();
-    bool any_team = false;
-    for (const ClassPlan& c : lp.classes) {
-        lp.team.push_back(team_pays(e, c.count) ? 1 : 0);
-        any_team = any_team || lp.team.back();
+    lp.team.assign(n, 0);
+    lp.tail.assign(n, 0u);
+    // The largest bodies first: the classes on teams share the schedulers.
+    double load = 0.0;
+    for (size_t c = n; c-- > 0;) {
+        const ClassPlan& k = lp.classes[c];
+        const double own = team_load(e, k.load, k.first_n, k.rows, k.mm);
+        if (pays(k, load + own)) {
+            lp.team[c] = 1;
+            load += own;
+        } else {
+            lp.tail[c] = tail_most(e, k.count, own, load, k.rows, k.mm);
+        }
     }
     lp.grids.assign(n, 0u);
+    const bool any_team = load > 0.0;
     if (!any_team) {
         lp.grids = class_grids(e, lp.classes, flags, rate);
     }
-    lp.tail = tail_most(e, pack->count);
     lp.slots_at.assign(n, 0);
     lp.tail_at.assign(n, 0);
     for (size_t c = 0; c < n; c++) {
@@ -354,7 +424,7 @@ ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, in
         lp.slots_at[c] = lp.scratch;
         lp.scratch += (scratch_bytes(lp.grids[c], k.rows, k.mm, false) + 255u) & ~(size_t)255u;
         lp.tail_at[c] = lp.scratch;
-        if (lp.tail) lp.scratch += cek::tail_bytes(k.rows, k.mm, lp.tail);
+        if (lp.tail[c]) lp.scratch += cek::tail_bytes(k.rows, k.mm, lp.tail[c]);
     }
     return CE_OK;
 }
@@ -406,7 +476,7 @@ ce_status launch_classes(ce_engine* e, const LaunchPlan& lp, cek::KernelArgs a, 
             }
             a.scratch = reinterpret_cast<float4*>(static_cast<char*>(scratch) + lp.slots_at[c]);
             const cek::LaunchSpec ls{k.rows, k.mm, flags, false, rate, lp.grids[c], cek::kBlock, on};
-            const ce_status s = launch_lanes(e, ls, a, p, static_cast<char*>(scratch) + lp.tail_at[c], lp.tail);
+            const ce_status s = launch_lanes(e, ls, a, p, static_cast<char*>(scratch) + lp.tail_at[c], lp.tail[c]);
             if (s != CE_OK) return s;
         }
     }
@@ -694,11 +764,8 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
     }
     std::vector<ClassPlan> plans;
     if ((s = plan_classes(pack, plans)) != CE_OK) return s;
-    unsigned rows = 2, mm = 0;
-    for (const ClassPlan& c : plans) {
-        rows = std::max(rows, c.rows);
-        mm = std::max(mm, c.mm);
-    }
+    const ClassPlan all = whole(plans);
+    const unsigned rows = all.rows, mm = all.mm;
     const uint32_t flags = ce_world_flags(w);
     const int rate = (int)ce::world_rate(*w);
     const uint32_t stride = ce_frame_stride(mm);
@@ -741,7 +808,7 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
     a.mm = mm;
     a.frames_per_creature = per;
     a.chunk_k = 1;
-    if (team_pays(e, pack->count)) {
+    if (team_pays(e, pack->count, team_load(e, all.load, rows, rows, mm), rows, mm, flags, true, rate)) {
         const cek::TeamSpec ts{flags, rate, cek::team_blocks(rows, a.count), (unsigned)e->sms, nullptr};
         CE_TRY(cek::launch_team_record(ts, a, p), "record launch");
     } else {
@@ -773,13 +840,20 @@ size_t slots_part(ce_engine* e, uint32_t world_flags, uint32_t rate, uint32_t ma
     if (e->opened_ctas) take(e->opened_ctas);
     return (scratch_bytes(grid, max_nodes, max_muscles, false) + 255u) & ~(size_t)255u;
 }
+// Only the largest body is known here: every creature is taken for one.
+double device_load(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_t max_muscles) {
+    return team_load(e, (double)count * team_cost(max_nodes, max_muscles), 0u, max_nodes, max_muscles);
+}
+unsigned device_tail(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_t max_muscles) {
+    return tail_most(e, count, device_load(e, count, max_nodes, max_muscles), 0.0, max_nodes, max_muscles);
+}
 }  // namespace
 
 extern "C" size_t ce_advance_scratch_bytes(ce_engine* e, uint32_t world_flags, uint32_t rate, uint32_t max_nodes,
                                            uint32_t max_muscles, uint32_t count) {
     if (!e || max_nodes < 2 || max_nodes > CE_MAX_NODES || max_muscles > CE_MAX_MUSCLES) return 0;
     if (rate != 60 && rate != 120) return 0;
-    const unsigned most = tail_most(e, count);
+    const unsigned most = device_tail(e, count, max_nodes, max_muscles);
     return slots_part(e, world_flags, rate, max_nodes, max_muscles) + cek::bucket_bytes(count) +
            (most ? cek::tail_bytes(max_nodes, max_muscles, most) : 0);
 }
@@ -830,7 +904,8 @@ ce_status advance_device(ce_engine* e, const uint32_t* records, const float* mus
         a.cells = cells;
         a.niche = *niche;
     }
-    if (team_pays(e, params->count)) {
+    if (team_pays(e, a.count, device_load(e, a.count, max_nodes, max_muscles), max_nodes, max_muscles, world_flags, false,
+                  (int)rate)) {
         const cek::TeamSpec ts{world_flags, (int)rate, cek::team_blocks(max_nodes, a.count), (unsigned)e->sms, st};
         CE_TRY(cek::launch_team(ts, a, *params), "advance launch");
         return CE_OK;
@@ -838,7 +913,7 @@ ce_status advance_device(ce_engine* e, const uint32_t* records, const float* mus
     const cek::LaunchSpec ls{max_nodes, max_muscles, world_flags, false, (int)rate, grid, cek::kBlock, st};
     char* const tail = static_cast<char*>(scratch) + slots_part(e, world_flags, rate, max_nodes, max_muscles) +
                        cek::bucket_bytes(params->count);
-    return launch_lanes(e, ls, a, *params, tail, tail_most(e, params->count));
+    return launch_lanes(e, ls, a, *params, tail, device_tail(e, a.count, max_nodes, max_muscles));
 }
 }  // namespace
 
@@ -877,6 +952,7 @@ struct ce_tape {
     cudaEvent_t start = nullptr, stop = nullptr;
     size_t count = 0;
     unsigned rows = 2, mm = 0, ckpts = 0, grid = 1;
+    double load = 0.0;  // team_load of the batch
     uint32_t flags = 0;
     int rate = 60;
     ce_params params{};
@@ -951,10 +1027,10 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     t->engine = e;
     t->count = pack->count;
     t->flags = flags;
-    for (const ClassPlan& c : plans) {
-        t->rows = std::max(t->rows, c.rows);
-        t->mm = std::max(t->mm, c.mm);
-    }
+    const ClassPlan all = whole(plans);
+    t->rows = all.rows;
+    t->mm = all.mm;
+    t->load = team_load(e, all.load, 0u, all.rows, all.mm);
     t->rate = (int)ce::world_rate(*w);
     if (cek::adjoint_smem_bytes(t->rows, t->mm, cek::kBlock) > e->smem_optin) {
         const std::string why = "ce_forward: bodies of " + std::to_string(t->rows) + " nodes and " +
@@ -1008,8 +1084,8 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
     cek::LaunchSpec ls{t->rows, t->mm, flags, false, t->rate, t->grid, cek::kBlock, st};
     const cek::TeamSpec ts{flags, t->rate, cek::team_blocks(t->rows, a.count), (unsigned)e->sms, st};
-    if ((s = cuda_status(team_pays(e, a.count) ? cek::launch_team_ckpt(ts, a, t->params)
-                                               : cek::launch_forward_ckpt(ls, a, t->params),
+    const bool team = team_pays(e, a.count, t->load, t->rows, t->mm, flags, false, t->rate);
+    if ((s = cuda_status(team ? cek::launch_team_ckpt(ts, a, t->params) : cek::launch_forward_ckpt(ls, a, t->params),
                          "forward launch")) ||
         (s = cuda_status(cudaEventRecord(t->stop, st), "cudaEventRecord")) ||
         (s = tape_time(t, &t->forward_seconds))) {
@@ -1065,7 +1141,8 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
     }
     const size_t needed = (t->count + cek::kBlock - 1) / cek::kBlock;
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min(needed, (size_t)per_sm * t->engine->sms));
-    const bool team = team_back_pays(t->engine, t->count);
+    const bool team = team_back_pays(t->engine, t->count, t->load, t->rows, t->mm,
+                                     (size_t)per_sm * t->engine->sms * cek::kBlock);
     unsigned blocks = 0;
     if (team) {
         CE_TRY(cek::team_adjoint_blocks(t->rows, t->mm, t->flags, t->rate, (unsigned)t->engine->sms, t->count, &blocks),
@@ -1340,10 +1417,10 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
     ce_wave_pack wp{lanes.data(), lanes_len, muscles.data(), mus_len, heads.data(), n};
     std::vector<ClassPlan> plans;
     if ((s = plan_classes(&wp, plans)) != CE_OK) return fail(s);
-    for (const ClassPlan& c : plans) {
-        a->rows = std::max(a->rows, c.rows);
-        a->mm = std::max(a->mm, c.mm);
-    }
+    const ClassPlan all = whole(plans);
+    a->rows = all.rows;
+    a->mm = all.mm;
+    const double load = team_load(e, all.load, 0u, all.rows, all.mm);
     if (cek::adjoint_smem_bytes(a->rows, a->mm, cek::kBlock) > e->smem_optin) {
         set_error("ce_ascent_open: bodies too large for the backward pass's shared memory");
         return fail(CE_ERR_UNSUPPORTED);
@@ -1365,7 +1442,8 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
     }
     const unsigned bgrid =
         (unsigned)std::max<size_t>(1, std::min((n + cek::kBlock - 1) / cek::kBlock, (size_t)per_sm * e->sms));
-    const bool team_back = team_back_pays(e, n);
+    const bool team = team_pays(e, n, load, a->rows, a->mm, flags, false, a->rate);
+    const bool team_back = team_back_pays(e, n, load, a->rows, a->mm, (size_t)per_sm * e->sms * cek::kBlock);
     unsigned bblocks = 0;
     if (team_back && (s = cuda_status(cek::team_adjoint_blocks(a->rows, a->mm, flags, a->rate, (unsigned)e->sms, n, &bblocks),
                                       "backward launch")) != CE_OK) {
@@ -1439,7 +1517,7 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         if (ce == cudaSuccess) ce = cudaMemsetAsync(a->d_ends.ptr, 0, n * 4, st);
         const cek::TeamSpec ts{flags, a->rate, cek::team_blocks(a->rows, n), (unsigned)e->sms, st};
         if (ce == cudaSuccess)
-            ce = team_pays(e, n) ? cek::launch_team_ckpt(ts, ka, a->params) : cek::launch_forward_ckpt(fs, ka, a->params);
+            ce = team ? cek::launch_team_ckpt(ts, ka, a->params) : cek::launch_forward_ckpt(fs, ka, a->params);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(a->d_grads.ptr, 0, n * per_grad * 4, st);
         if (ce == cudaSuccess) ce = cek::launch_bucket(heads_d, 0u, (uint32_t)n, bk, st);
         const cek::TeamSpec tb{flags, a->rate, bblocks, (unsigned)e->sms, st};
@@ -1473,7 +1551,7 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         ka.ends = nullptr;
         const cek::LaunchSpec ls{a->rows, a->mm, flags, false, a->rate, fgrid, cek::kBlock, st};
         const cek::TeamSpec ts{flags, a->rate, cek::team_blocks(a->rows, n), (unsigned)e->sms, st};
-        ce = team_pays(e, n) ? cek::launch_team(ts, ka, a->params) : cek::launch_advance(ls, ka, a->params);
+        ce = team ? cek::launch_team(ts, ka, a->params) : cek::launch_advance(ls, ka, a->params);
     }
     cudaGraph_t graph = nullptr;
     const ce_status end = cuda_status(cudaStreamEndCapture(st, &graph), "cudaStreamEndCapture");

@@ -174,6 +174,8 @@ struct TeamSpec {
     unsigned share = 1u;  // leave the rest of the GPU to another launch: 1 / share of the blocks that fit
 };
 unsigned team_blocks(unsigned rows, size_t count);
+// Shared memory of a block for bodies of `first_n` to `rows` nodes.
+size_t team_smem_bytes(unsigned first_n, unsigned rows, unsigned mm);
 cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 cudaError_t launch_team_record(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_params& p);

@@ -16,6 +16,15 @@ unsigned team_blocks(unsigned rows, size_t count) {
     return (unsigned)(blocks < 0x7fffffffu ? blocks : 0x7fffffffu);
 }
 
+size_t team_smem_bytes(unsigned first_n, unsigned rows, unsigned mm) {
+    KernelArgs a{};
+    a.queues = kQueues;
+    a.first_n = first_n;
+    a.rows = rows;
+    a.mm = mm;
+    return (size_t)team_warp_bytes(a, false) * (kTeamBlock / 32u);
+}
+
 namespace {
 size_t align256(size_t b) { return (b + 255u) & ~(size_t)255u; }
 }  // namespace

@@ -11,8 +11,7 @@ namespace cek {
 inline unsigned team_warp_bytes(const KernelArgs& a, bool record) {
     unsigned most = 0u;
     for (unsigned lanes = 8u; lanes <= 32u; lanes *= 2u) {
-        const bool used = a.resume ? lanes <= team_lanes(a.rows)
-                          : a.queues == 0u ? lanes == team_lanes(a.rows)
+        const bool used = a.queues == 0u ? lanes == team_lanes(a.rows)
                                          : lanes >= team_lanes(a.first_n) && lanes <= team_lanes(a.rows);
         const unsigned bytes = 32u / lanes * TeamLayout::make(lanes, a.mm, record).bytes;
         if (used && bytes > most) most = bytes;

@@ -1,0 +1,54 @@
+"""A launch goes on teams of lanes only where that is the faster: against an
+engine that keeps one creature a lane, on bodies of one size at counts where
+their number alone would put them on teams. Teams take 1.5 to 2.5 times as
+long there."""
+import numpy as np
+import pytest
+
+import evolution_simulator_gpu_b200 as ce
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lanes():
+    pytest.importorskip("torch")
+    with ce.Engine(0, teams=2) as e:
+        yield e
+
+
+def bodies(nodes, muscles, count):
+    return ce.generate(ce.GenSpecPy(seed=9, min_nodes=nodes, max_nodes=nodes, muscle_rule=1, min_muscles=muscles,
+                                    max_muscles=muscles, joint_lo_deg=30.0, joint_hi_deg=150.0), count)
+
+
+def bits(a):
+    return np.ascontiguousarray(a).view(np.uint32)
+
+
+@pytest.mark.parametrize("nodes,muscles,count", [(3, 1, 24_576), (3, 1, 28_000), (9, 1, 24_576), (17, 8, 24_576),
+                                                 (17, 8, 28_000), (24, 1, 24_576)])
+def test_trials(engine, lanes, nodes, muscles, count):
+    w = ce.make_world(duration=1.5)
+    wave = ce.pack(bodies(nodes, muscles, count), w)
+    a, b = engine.run(wave, w)[0], lanes.run(wave, w)[0]
+    assert (bits(a) == bits(b)).all()
+    mine, theirs = (min(e.run(wave, w)[1] for _ in range(3)) for e in (engine, lanes))
+    assert mine < 1.15 * theirs
+
+
+@pytest.mark.parametrize("nodes,muscles,count", [(3, 1, 16_384), (9, 8, 32_768), (17, 8, 32_768)])
+def test_backward_runs(engine, lanes, nodes, muscles, count):
+    w = ce.make_world(duration=0.5)
+    wave = ce.pack(bodies(nodes, muscles, count), w)
+    took, grads = [], []
+    for e in (engine, lanes):
+        with e.forward(wave, w) as tape:
+            grads.append(tape.backward())
+            seconds = []
+            for _ in range(2):
+                tape.backward()
+                seconds.append(tape.seconds[1])
+            took.append(min(seconds))
+    assert (bits(grads[0]) == bits(grads[1])).all()
+    assert took[0] < 1.15 * took[1]
