@@ -100,6 +100,7 @@ struct Slot {
     bool busy = false;
     uint64_t ticket = 0;
     size_t count = 0;
+    double load = 0.0;  // team_load of the submission
     cudaStream_t stream = nullptr, side = nullptr;  // side: the second class
     cudaEvent_t start = nullptr, stop = nullptr, done = nullptr, joined = nullptr, bucketed = nullptr;
     DeviceBuf d_lanes, d_muscles, d_heads, d_results, d_buckets, d_scratch;
@@ -257,11 +258,15 @@ bool team_pays(ce_engine* e, size_t count, double load, unsigned rows, unsigned 
 }
 // Creatures left at which a lane launch of `load` hands its trials over to
 // teams: three quarters of those that teams pay for beside `others` (ns a
-// substep) on teams already, each taken for an average one; 0 for none.
-unsigned tail_most(const ce_engine* e, size_t count, double load, double others, unsigned rows, unsigned mm) {
+// substep), each taken for an average one.
+unsigned tail_fit(const ce_engine* e, size_t count, double load, double others, unsigned rows, unsigned mm) {
     if (!e->teams || e->tuning || count == 0) return 0u;
-    const double most = std::min(0.75 * lane_chain(rows, mm) * (double)count / (load + others), (double)kTeamMost);
-    return (double)count > most ? (unsigned)most : 0u;
+    return (unsigned)std::min(0.75 * lane_chain(rows, mm) * (double)count / (load + others), (double)kTeamMost);
+}
+// 0 for none: a launch that is no larger starts on teams, or stays on lanes.
+unsigned tail_most(const ce_engine* e, size_t count, double load, double others, unsigned rows, unsigned mm) {
+    const unsigned most = tail_fit(e, count, load, others, rows, mm);
+    return count > most ? most : 0u;
 }
 // Whether a backward run goes on teams: the same trade, 6 times the forward
 // load against 5 times its chain, and again for each round of `lanes` (ms a
@@ -371,6 +376,7 @@ struct LaunchPlan {
     std::vector<size_t> slots_at, tail_at;   // offsets in the scratch
     std::vector<unsigned> tail;              // creatures that each lane launch hands over
     size_t scratch = 0;
+    double load = 0.0;                       // team_load of the batch
 };
 
 // All classes as one, for what serves every node count in one launch.
@@ -386,37 +392,57 @@ ClassPlan whole(const std::vector<ClassPlan>& plans) {
     return all;
 }
 
-ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, int rate, LaunchPlan& lp) {
+// Which classes of a batch go on teams, beside `others` (team_load of the
+// submissions in flight, which share the schedulers with it). A stream of
+// batches goes on teams while together they take those no longer than a
+// lane's chain; small batches up to 1.75 chains, since lanes take each of
+// them a whole one. Other batches of a stream go on lanes in all their
+// classes, with their share of the tail (8 batches through 4 slots, 4 s, ms on
+// lanes / each as if alone / so: calm, 8,192 game bodies 155 / 108 / 108,
+// 16,384 187 / 192 / 170, 24,576 229 / 278 / 227, 16,384 small bodies 86 / 126
+// / 82; in the effects world, where most fall, 227 / 116 / 116 for 8,192
+// refine bodies, 198 / 107 / 102 for 16,384 game bodies). The tails still cost
+// a stream of large batches whose creatures all stand: 24,576 refine bodies in
+// thick air 303 / 467 / 327.
+void plan_routes(ce_engine* e, const std::vector<ClassPlan>& classes, uint32_t flags, int rate, double others,
+                 LaunchPlan& lp) {
     lp = LaunchPlan{};
-    ce_status s = plan_classes(pack, lp.classes, e->small_body);
-    if (s != CE_OK || lp.classes.empty()) return s;
+    lp.classes = classes;
     const auto pays = [&](const ClassPlan& c, double load) {
         return team_pays(e, c.count, load, c.rows, c.mm, flags, false, rate);
     };
-    const ClassPlan all = whole(lp.classes);
-    if (pays(all, team_load(e, all.load, all.first_n, all.rows, all.mm))) lp.classes.assign(1, all);
+    const ClassPlan all = whole(classes);
+    lp.load = team_load(e, all.load, all.first_n, all.rows, all.mm);
+    const double chain = lane_chain(all.rows, all.mm);
+    const bool small = lp.load <= 0.45 * chain && others + lp.load <= 1.75 * chain;
+    const bool one = pays(all, small ? lp.load : others + lp.load);
+    if (one) lp.classes.assign(1, all);
     const size_t n = lp.classes.size();
     lp.team.assign(n, 0);
     lp.tail.assign(n, 0u);
     // The largest bodies first: the classes on teams share the schedulers.
-    double load = 0.0;
+    double load = others;
     for (size_t c = n; c-- > 0;) {
         const ClassPlan& k = lp.classes[c];
         const double own = team_load(e, k.load, k.first_n, k.rows, k.mm);
-        if (pays(k, load + own)) {
+        if (one || (others == 0.0 && pays(k, load + own))) {
             lp.team[c] = 1;
             load += own;
         } else {
             lp.tail[c] = tail_most(e, k.count, own, load, k.rows, k.mm);
         }
     }
+}
+
+// Grids, and where each class's slots and tail are in the scratch.
+void plan_scratch(ce_engine* e, uint32_t flags, int rate, LaunchPlan& lp) {
+    const size_t n = lp.classes.size();
+    const bool any_team = std::find(lp.team.begin(), lp.team.end(), 1) != lp.team.end();
     lp.grids.assign(n, 0u);
-    const bool any_team = load > 0.0;
-    if (!any_team) {
-        lp.grids = class_grids(e, lp.classes, flags, rate);
-    }
+    if (!any_team) lp.grids = class_grids(e, lp.classes, flags, rate);
     lp.slots_at.assign(n, 0);
     lp.tail_at.assign(n, 0);
+    lp.scratch = 0;
     for (size_t c = 0; c < n; c++) {
         if (lp.team[c]) continue;
         const ClassPlan& k = lp.classes[c];
@@ -425,6 +451,36 @@ ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, in
         lp.scratch += (scratch_bytes(lp.grids[c], k.rows, k.mm, false) + 255u) & ~(size_t)255u;
         lp.tail_at[c] = lp.scratch;
         if (lp.tail[c]) lp.scratch += cek::tail_bytes(k.rows, k.mm, lp.tail[c]);
+    }
+}
+
+// The plan of a batch beside `others`. Its scratch (`reserve` bytes) is as
+// large as the batch needs beside any others, so a slot's area does not grow
+// with the timing of its neighbours while they run.
+ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, int rate, double others, LaunchPlan& lp,
+                      size_t* reserve) {
+    lp = LaunchPlan{};
+    *reserve = 0;
+    std::vector<ClassPlan> classes;
+    ce_status s = plan_classes(pack, classes, e->small_body);
+    if (s != CE_OK || classes.empty()) return s;
+    plan_routes(e, classes, flags, rate, 0.0, lp);
+    plan_scratch(e, flags, rate, lp);
+    *reserve = lp.scratch;
+    if (e->slots.size() < 2) return CE_OK;
+    // All on lanes, with the longest tails.
+    LaunchPlan lanes;
+    lanes.classes = classes;
+    lanes.team.assign(classes.size(), 0);
+    for (const ClassPlan& k : classes) {
+        const double own = team_load(e, k.load, k.first_n, k.rows, k.mm);
+        lanes.tail.push_back(std::min(k.count, tail_fit(e, k.count, own, 0.0, k.rows, k.mm)));
+    }
+    plan_scratch(e, flags, rate, lanes);
+    *reserve = std::max(*reserve, lanes.scratch);
+    if (others > 0.0) {
+        plan_routes(e, classes, flags, rate, others, lp);
+        plan_scratch(e, flags, rate, lp);
     }
     return CE_OK;
 }
@@ -649,13 +705,19 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
     const int rate = (int)ce::world_rate(*w);
     ce_params p;
     ce_make_params(w, 0, (uint32_t)pack->count, 0, &p);
+    double others = 0.0;
+    for (const size_t i : e->pending) {
+        if (cudaEventQuery(e->slots[i].done) != cudaSuccess) others += e->slots[i].load;
+    }
+    cudaGetLastError();
     LaunchPlan lp;
-    if ((s = plan_launch(e, pack, flags, rate, lp)) != CE_OK) return s;
+    size_t reserve = 0;
+    if ((s = plan_launch(e, pack, flags, rate, others, lp, &reserve)) != CE_OK) return s;
     const size_t lanes_b = pack->lanes_len * 4, mus_b = pack->muscles_len * 4, heads_b = pack->count * 32;
     const size_t res_b = pack->count * sizeof(ce_result);
     if ((s = sl.d_lanes.ensure(lanes_b)) || (s = sl.d_muscles.ensure(mus_b)) || (s = sl.d_heads.ensure(heads_b)) ||
         (s = sl.d_buckets.ensure(cek::bucket_bytes(pack->count))) || (s = sl.d_results.ensure(res_b)) ||
-        (s = sl.d_scratch.ensure(lp.scratch)) || (s = sl.h_upload.ensure(lanes_b + mus_b + heads_b)) ||
+        (s = sl.d_scratch.ensure(reserve)) || (s = sl.h_upload.ensure(lanes_b + mus_b + heads_b)) ||
         (s = sl.h_results.ensure(res_b))) {
         return s;
     }
@@ -684,6 +746,7 @@ extern "C" ce_status ce_submit(ce_engine* e, const ce_wave_pack* pack, const ce_
     CE_TRY(cudaEventRecord(sl.done, st), "cudaEventRecord");
     sl.busy = true;
     sl.count = pack->count;
+    sl.load = lp.load;
     sl.ticket = e->next_ticket++;
     sl.submitted = std::chrono::steady_clock::now();
     e->pending.push_back(si);
@@ -1680,7 +1743,8 @@ extern "C" ce_status ce_graph_open(ce_engine* e, const ce_wave_pack* packs, uint
             set_error("ce_graph_open: empty generation");
             return fail(CE_ERR_INVALID);
         }
-        if ((s = plan_launch(e, pack, flags, rate, plans[k])) != CE_OK) return fail(s);
+        size_t reserve = 0;
+        if ((s = plan_launch(e, pack, flags, rate, 0.0, plans[k], &reserve)) != CE_OK) return fail(s);
         scratch_need = std::max(scratch_need, plans[k].scratch);
         ce_graph::Gen& gen = g->gens[k];
         gen.count = pack->count;

@@ -2,10 +2,13 @@
 engine that keeps one creature a lane, on bodies of one size at counts where
 their number alone would put them on teams. Teams take 1.5 to 2.5 times as
 long there."""
+import time
+
 import numpy as np
 import pytest
 
 import evolution_simulator_gpu_b200 as ce
+from evolution_simulator_gpu_b200.configs import WORKLOADS
 
 pytestmark = pytest.mark.gpu
 
@@ -51,4 +54,31 @@ def test_backward_runs(engine, lanes, nodes, muscles, count):
                 seconds.append(tape.seconds[1])
             took.append(min(seconds))
     assert (bits(grads[0]) == bits(grads[1])).all()
+    assert took[0] < 1.15 * took[1]
+
+
+def test_a_stream_of_batches(engine, lanes):
+    """Four submissions in flight share the schedulers: each as if it were
+    alone on teams takes 1.4 times as long as on lanes."""
+    w = ce.make_world(duration=4.0)
+    spec = WORKLOADS["small"].spec
+    waves = [ce.pack(ce.generate(spec, 16_384, first=16_384 * k), w) for k in range(4)]
+
+    def stream(e):
+        out, sent = [], 0
+        start = time.perf_counter()
+        while len(out) < 8:
+            while sent < 8 and e.free_slots():
+                e.submit(waves[sent % 4], w)
+                sent += 1
+            out.append(e.poll(60.0)[1])
+        return time.perf_counter() - start, out
+
+    took, results = [], []
+    for e in (engine, lanes):
+        stream(e)
+        runs = [stream(e) for _ in range(3)]
+        took.append(min(r[0] for r in runs))
+        results.append(runs[0][1])
+    assert all((bits(a) == bits(b)).all() for a, b in zip(*results))
     assert took[0] < 1.15 * took[1]
