@@ -94,6 +94,7 @@ struct ClassPlan {
     uint32_t mm;               // most muscles in the class
     double work;               // estimated arithmetic of a substep of all its creatures
     double load;               // a substep of all its creatures on teams (team_load), ns
+    uint32_t sized[3];         // creatures of each team size
 };
 
 struct Slot {
@@ -351,7 +352,7 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
         cost_n[n] += team_cost(n, m);
     }
     for (int big = 0; big < 2; big++) {
-        ClassPlan c{0, 0, 0, 2, 0, 0.0, 0.0};
+        ClassPlan c{0, 0, 0, 2, 0, 0.0, 0.0, {0, 0, 0}};
         for (unsigned n = 2; n <= CE_MAX_NODES; n++) {
             if (per_n[n] == 0 || (n > small_body) != (big != 0)) continue;
             if (c.count == 0) c.first_n = n;
@@ -361,6 +362,7 @@ ce_status plan_classes(const ce_wave_pack* pack, std::vector<ClassPlan>& plans, 
             c.mm = std::max(c.mm, mm_n[n]);
             c.work += work_n[n];
             c.load += cost_n[n];
+            c.sized[n <= 8u ? 0 : n <= 16u ? 1 : 2] += (uint32_t)per_n[n];
         }
         if (c.count) plans.push_back(c);
     }
@@ -388,8 +390,15 @@ ClassPlan whole(const std::vector<ClassPlan>& plans) {
         all.mm = std::max(all.mm, plans[c].mm);
         all.count += plans[c].count;
         all.load += plans[c].load;
+        for (int g = 0; g < 3; g++) all.sized[g] += plans[c].sized[g];
     }
     return all;
+}
+// Warps that run all of a plan's creatures on teams at once.
+size_t team_warps(const ClassPlan& c) {
+    size_t warps = 0;
+    for (unsigned g = 0; g < 3; g++) warps += (c.sized[g] + (4u >> g) - 1u) / (4u >> g);
+    return warps;
 }
 
 // Which classes of a batch go on teams, beside `others` (team_load of the
@@ -844,12 +853,14 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
     // Frames are indexed by packed creature, so any grid records them; one
     // block of lanes per 128 creatures, up to what the GPU holds at once.
     const unsigned grid = grid_for(e, rows, mm, flags, true, rate, pack->count);
+    const bool team = team_pays(e, pack->count, team_load(e, all.load, rows, rows, mm), rows, mm, flags, true, rate);
     const size_t lanes_b = pack->lanes_len * 4, mus_b = pack->muscles_len * 4, heads_b = pack->count * 32;
     const size_t res_b = pack->count * sizeof(ce_result);
     if ((s = e->rec_frames.ensure(frame_floats * 4)) || (s = e->rec_staging.ensure(frame_floats * 4)) ||
         (s = e->rec_lanes.ensure(lanes_b)) ||
         (s = e->rec_muscles.ensure(mus_b)) || (s = e->rec_heads.ensure(heads_b)) || (s = e->rec_results.ensure(res_b)) ||
-        (s = e->rec_counter.ensure(4)) || (s = e->rec_scratch.ensure(scratch_bytes(grid, rows, mm, true)))) {
+        (s = e->rec_counter.ensure(4)) ||
+        (!team && (s = e->rec_scratch.ensure(scratch_bytes(grid, rows, mm, true))))) {
         return s;
     }
     CE_TRY(cudaMemcpy(e->rec_lanes.ptr, pack->lanes, lanes_b, cudaMemcpyHostToDevice), "cudaMemcpy");
@@ -871,7 +882,7 @@ extern "C" ce_status ce_record(ce_engine* e, const ce_wave_pack* pack, const ce_
     a.mm = mm;
     a.frames_per_creature = per;
     a.chunk_k = 1;
-    if (team_pays(e, pack->count, team_load(e, all.load, rows, rows, mm), rows, mm, flags, true, rate)) {
+    if (team) {
         const cek::TeamSpec ts{flags, rate, cek::team_blocks(rows, a.count), (unsigned)e->sms, nullptr};
         CE_TRY(cek::launch_team_record(ts, a, p), "record launch");
     } else {
@@ -1016,6 +1027,7 @@ struct ce_tape {
     size_t count = 0;
     unsigned rows = 2, mm = 0, ckpts = 0, grid = 1;
     double load = 0.0;  // team_load of the batch
+    size_t warps = 0;   // team_warps of the batch
     uint32_t flags = 0;
     int rate = 60;
     ce_params params{};
@@ -1094,6 +1106,7 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     t->rows = all.rows;
     t->mm = all.mm;
     t->load = team_load(e, all.load, 0u, all.rows, all.mm);
+    t->warps = team_warps(all);
     t->rate = (int)ce::world_rate(*w);
     if (cek::adjoint_smem_bytes(t->rows, t->mm, cek::kBlock) > e->smem_optin) {
         const std::string why = "ce_forward: bodies of " + std::to_string(t->rows) + " nodes and " +
@@ -1119,11 +1132,12 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     const size_t res_b = pack->count * sizeof(ce_result);
     const size_t ckpt_b = pack->count * (size_t)t->ckpts * cek::checkpoint_floats(t->rows, t->mm) * 4;
     t->grid = grid_for(e, t->rows, t->mm, flags, false, t->rate, pack->count);
+    const bool team = team_pays(e, pack->count, t->load, t->rows, t->mm, flags, false, t->rate);
     if ((s = t->d_lanes.ensure(lanes_b)) || (s = t->d_muscles.ensure(std::max<size_t>(mus_b, 4))) ||
         (s = t->d_heads.ensure(heads_b)) || (s = t->d_results.ensure(res_b)) ||
         (s = t->d_buckets.ensure(cek::bucket_bytes(pack->count))) || (s = t->d_ckpt.ensure(ckpt_b)) ||
         (s = t->d_ends.ensure(pack->count * 4)) ||
-        (s = t->d_scratch.ensure(scratch_bytes(t->grid, t->rows, t->mm, false)))) {
+        (!team && (s = t->d_scratch.ensure(scratch_bytes(t->grid, t->rows, t->mm, false))))) {
         return fail(s);
     }
     cudaStream_t st = t->stream;
@@ -1147,7 +1161,6 @@ extern "C" ce_status ce_forward(ce_engine* e, const ce_wave_pack* pack, const ce
     a.scratch = static_cast<float4*>(t->d_scratch.ptr);
     cek::LaunchSpec ls{t->rows, t->mm, flags, false, t->rate, t->grid, cek::kBlock, st};
     const cek::TeamSpec ts{flags, t->rate, cek::team_blocks(t->rows, a.count), (unsigned)e->sms, st};
-    const bool team = team_pays(e, a.count, t->load, t->rows, t->mm, flags, false, t->rate);
     if ((s = cuda_status(team ? cek::launch_team_ckpt(ts, a, t->params) : cek::launch_forward_ckpt(ls, a, t->params),
                          "forward launch")) ||
         (s = cuda_status(cudaEventRecord(t->stop, st), "cudaEventRecord")) ||
@@ -1208,7 +1221,7 @@ ce_status backward(ce_tape* t, const float* dl_dfitness, float* grads, size_t ca
                                      (size_t)per_sm * t->engine->sms * cek::kBlock);
     unsigned blocks = 0;
     if (team) {
-        CE_TRY(cek::team_adjoint_blocks(t->rows, t->mm, t->flags, t->rate, (unsigned)t->engine->sms, t->count, &blocks),
+        CE_TRY(cek::team_adjoint_blocks(t->rows, t->mm, t->flags, t->rate, (unsigned)t->engine->sms, t->warps, &blocks),
                "backward launch");
     }
     const size_t slot_b = team ? 0 : cek::adjoint_slot_bytes(grid, t->rows, t->mm);
@@ -1508,7 +1521,7 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
     const bool team = team_pays(e, n, load, a->rows, a->mm, flags, false, a->rate);
     const bool team_back = team_back_pays(e, n, load, a->rows, a->mm, (size_t)per_sm * e->sms * cek::kBlock);
     unsigned bblocks = 0;
-    if (team_back && (s = cuda_status(cek::team_adjoint_blocks(a->rows, a->mm, flags, a->rate, (unsigned)e->sms, n, &bblocks),
+    if (team_back && (s = cuda_status(cek::team_adjoint_blocks(a->rows, a->mm, flags, a->rate, (unsigned)e->sms, team_warps(all), &bblocks),
                                       "backward launch")) != CE_OK) {
         return fail(s);
     }
@@ -1530,7 +1543,7 @@ extern "C" ce_status ce_ascent_open(ce_engine* e, const ce_population* pop, cons
         (s = up(a->d_heads, heads.data(), n * 32)) || (s = a->d_buckets.ensure(cek::bucket_bytes(n))) ||
         (s = a->d_ckpt.ensure(n * (size_t)a->ckpts * cek::checkpoint_floats(a->rows, a->mm) * 4)) ||
         (s = a->d_ends.ensure(n * 4)) ||
-        (s = a->d_scratch.ensure(std::max(scratch_bytes(fgrid, a->rows, a->mm, false),
+        (s = a->d_scratch.ensure(std::max(team ? 0 : scratch_bytes(fgrid, a->rows, a->mm, false),
                                           team_back ? 0 : cek::adjoint_slot_bytes(bgrid, a->rows, a->mm)))) ||
         (s = a->d_tape.ensure(team_back ? cek::team_adjoint_tape_bytes(bblocks, a->rows, a->mm)
                                         : cek::adjoint_tape_bytes(bgrid, a->rows, a->mm))) ||

@@ -180,10 +180,11 @@ cudaError_t launch_team(const TeamSpec& s, const KernelArgs& a, const ce_params&
 cudaError_t launch_team_record(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 cudaError_t launch_team_ckpt(const TeamSpec& s, const KernelArgs& a, const ce_params& p);
 
-// The backward run on teams (team_adjoint.cu): its blocks, the bytes of its
-// segment tapes and its launch (TeamSpec::blocks of them).
+// The backward run on teams (team_adjoint.cu): its blocks for `warps` warps of
+// teams, the bytes of its segment tapes and its launch (TeamSpec::blocks of
+// them).
 constexpr unsigned kTeamAdjointMinBlocks = 4;
-cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t count,
+cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t warps,
                                 unsigned* blocks);
 size_t team_adjoint_tape_bytes(unsigned blocks, unsigned rows, unsigned mm);
 cudaError_t launch_team_adjoint(const TeamSpec& s, const KernelArgs& a, const ce_params& p, float* tape, float* grads,

@@ -720,7 +720,7 @@ size_t team_adjoint_tape_bytes(unsigned blocks, unsigned rows, unsigned mm) {
     return (size_t)blocks * (kTeamBlock / 32u) * team_tape_warp_floats(rows, mm) * 4u;
 }
 
-cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t count,
+cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int rate, unsigned sms, size_t warps,
                                 unsigned* blocks) {
     const size_t smem = (size_t)team_adjoint_warp_bytes(2u, rows, mm) * (kTeamBlock / 32u);
     return with_gradient_world(flags, rate, [&](auto w, auto rt) -> cudaError_t {
@@ -731,8 +731,8 @@ cudaError_t team_adjoint_blocks(unsigned rows, unsigned mm, uint32_t flags, int 
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)kTeamBlock, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        const unsigned need = team_blocks(rows, count), full = (unsigned)per_sm * sms;
-        *blocks = need < full ? need : full;
+        const size_t need = (warps + kTeamBlock / 32u - 1u) / (kTeamBlock / 32u), full = (size_t)per_sm * sms;
+        *blocks = (unsigned)(need < 1u ? 1u : need < full ? need : full);
         return cudaSuccess;
     });
 }

@@ -82,3 +82,20 @@ def test_a_stream_of_batches(engine, lanes):
         results.append(runs[0][1])
     assert all((bits(a) == bits(b)).all() for a, b in zip(*results))
     assert took[0] < 1.15 * took[1]
+
+
+def test_a_backward_run_holds_tapes_for_its_teams_only(engine):
+    """1,000 bodies of up to 8 nodes, 4 to a warp, and one of more than 16: 251
+    warps of 1.2 MB, not one for every body because the largest fills one."""
+    import torch
+    w = ce.make_world(duration=0.5)
+    pop = ce.generate(WORKLOADS["effects"].spec, 3000)
+    nodes = pop.genomes["node_count"]
+    wave = ce.pack(pop.subset(np.concatenate([np.where(nodes <= 8)[0][:1000], np.where(nodes > 16)[0][:1]])), w)
+    assert len(wave) == 1001
+    with engine.forward(wave, w) as tape:
+        tape.backward()  # kernels and their local memory are loaded
+    free = torch.cuda.mem_get_info()[0]
+    with engine.forward(wave, w) as tape:
+        tape.backward()
+        assert free - torch.cuda.mem_get_info()[0] < 0.6e9
