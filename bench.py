@@ -41,10 +41,16 @@ WORKLOAD = "game"
 # Kernels of one device-entry call besides the creature kernel: the node-count
 # bucketing (count, scan, scatter) that builds the claim queues.
 BUCKET_KERNELS = 3
-# Creatures up to which a launch runs on teams of lanes, in one kernel; above,
-# each size class is a kernel of one creature a lane and the team kernel that
-# finishes its last trials.
-TEAM_MOST = 24576
+# Creatures from which every size class starts one creature a lane and ends on
+# teams of lanes, two kernels; with fewer a class may be one, and counts as one.
+TWO_KERNELS = 100_000
+SMALL_BODY = 12  # most nodes of the first size class
+
+
+def class_kernels(count):
+    return 2 if count >= TWO_KERNELS else int(count > 0)
+
+
 WORKLOAD_TEXT = ("3,000,000 seeded synthetic creatures (seed 1), 3-10 nodes, 2-24 muscles, calm flat world, "
                  "20 s trials at 60 steps/s x 16 substeps, FP32")
 
@@ -421,8 +427,7 @@ def run_engine(args):
     # End to end through the C ABI with host buffers.
     e2e_launches = 0
     nodes = wave.heads[:, 0] & 255
-    classes = 1 if len(wave) <= TEAM_MOST else sum(2 if n > TEAM_MOST else int(n > 0)
-                                                   for n in ((nodes <= 16).sum(), (nodes > 16).sum()))
+    classes = class_kernels((nodes <= SMALL_BODY).sum()) + class_kernels((nodes > SMALL_BODY).sum())
     h2d = wave.lanes.nbytes + wave.muscles.nbytes + wave.heads.nbytes + 4 * len(wave)
     d2h = len(wave) * ce.RESULT_DTYPE.itemsize
     eng.run(wave, world)  # buffers sized, pinned staging allocated
@@ -471,7 +476,7 @@ def run_engine(args):
             "parity": {"results_sha256": results_digest(res),
                        "compare_with": "the reference arm's reference_gpu.results_sha256: the reference kernel's "
                                        "results for the same generation in the same packed order"},
-            "gpu_launches": (BUCKET_KERNELS + (2 if len(wave) > TEAM_MOST else 1)) * args.steps, "gpu_launches_e2e": e2e_launches,
+            "gpu_launches": (BUCKET_KERNELS + class_kernels(len(wave))) * args.steps, "gpu_launches_e2e": e2e_launches,
             "roofline": roofline, "cpu_baseline": cpu, "clocks": clk, "adjoint": adjoint, "effects": effects,
             "f3": f3,
         }

@@ -264,11 +264,6 @@ unsigned tail_fit(const ce_engine* e, size_t count, double load, double others, 
     if (!e->teams || e->tuning || count == 0) return 0u;
     return (unsigned)std::min(0.75 * lane_chain(rows, mm) * (double)count / (load + others), (double)kTeamMost);
 }
-// 0 for none: a launch that is no larger starts on teams, or stays on lanes.
-unsigned tail_most(const ce_engine* e, size_t count, double load, double others, unsigned rows, unsigned mm) {
-    const unsigned most = tail_fit(e, count, load, others, rows, mm);
-    return count > most ? most : 0u;
-}
 // Whether a backward run goes on teams: the same trade, 6 times the forward
 // load against 5 times its chain, and again for each round of `lanes` (ms a
 // 1 s trial on teams / on lanes, calm: 8,192 bodies of 3 nodes 13.6 / 11.2, 9
@@ -401,6 +396,12 @@ size_t team_warps(const ClassPlan& c) {
     return warps;
 }
 
+// A substep of a class on lanes, which take its creatures in rounds (ns).
+double lane_time(ce_engine* e, const ClassPlan& k, uint32_t flags, int rate) {
+    const double lanes = (double)grid_for(e, k.rows, k.mm, flags, false, rate, (size_t)1 << 30) * cek::kBlock;
+    return lane_chain(k.rows, k.mm) * std::max(1.0, k.count / lanes);
+}
+
 // Which classes of a batch go on teams, beside `others` (team_load of the
 // submissions in flight, which share the schedulers with it). A stream of
 // batches goes on teams while together they take those no longer than a
@@ -417,29 +418,51 @@ void plan_routes(ce_engine* e, const std::vector<ClassPlan>& classes, uint32_t f
                  LaunchPlan& lp) {
     lp = LaunchPlan{};
     lp.classes = classes;
-    const auto pays = [&](const ClassPlan& c, double load) {
-        return team_pays(e, c.count, load, c.rows, c.mm, flags, false, rate);
-    };
     const ClassPlan all = whole(classes);
+    // Teams beside other teams have until the longest chain of them.
+    const auto pays = [&](const ClassPlan& c, double load, const ClassPlan& longest) {
+        return team_pays(e, c.count, load, longest.rows, longest.mm, flags, false, rate);
+    };
     lp.load = team_load(e, all.load, all.first_n, all.rows, all.mm);
     const double chain = lane_chain(all.rows, all.mm);
     const bool small = lp.load <= 0.45 * chain && others + lp.load <= 1.75 * chain;
-    const bool one = pays(all, small ? lp.load : others + lp.load);
+    const bool one = pays(all, small ? lp.load : others + lp.load, all);
     if (one) lp.classes.assign(1, all);
     const size_t n = lp.classes.size();
     lp.team.assign(n, 0);
     lp.tail.assign(n, 0u);
-    // The largest bodies first: the classes on teams share the schedulers.
+    // The largest bodies first: the classes on teams share the schedulers. One
+    // class goes on teams beside another on lanes where its own chain is the
+    // longer and the two together end within one and a half of it; else both
+    // go on lanes, which share the GPU the better the fuller it is (ms so /
+    // whenever a class alone would pay / never / before teams, 3 s: 60,000
+    // effects bodies 59 / 58 / 70 / 106, 200,000 of them 111 / 137 / 112 / 123,
+    // 40,000 of 3 to 24 nodes 92 / 108 / 92 / 111, 60,000 refine bodies 70 / 77
+    // / 70 / 79).
     double load = others;
     for (size_t c = n; c-- > 0;) {
         const ClassPlan& k = lp.classes[c];
-        const double own = team_load(e, k.load, k.first_n, k.rows, k.mm);
-        if (one || (others == 0.0 && pays(k, load + own))) {
+        const double own = team_load(e, k.load, k.first_n, k.rows, k.mm), chain = lane_chain(k.rows, k.mm);
+        double rest = 0.0;  // the other class's time on lanes
+        for (size_t o = 0; o < n; o++) {
+            if (o != c && !lp.team[o]) rest += lane_time(e, lp.classes[o], flags, rate);
+        }
+        if (one || (others == 0.0 && rest < chain && own + rest <= 1.5 * chain &&
+                    pays(k, load + own, load > 0.0 ? all : k))) {
             lp.team[c] = 1;
             load += own;
         } else {
-            lp.tail[c] = tail_most(e, k.count, own, load, k.rows, k.mm);
+            // With lanes of another class beside it a class keeps to lanes
+            // until half of it has ended.
+            const unsigned fit = tail_fit(e, k.count, own, load, k.rows, k.mm);
+            lp.tail[c] = n == 1 && k.count > fit ? fit : std::min(fit, k.count / 2u);
         }
+    }
+    // All on teams are one launch, whose warps go round by the classes' work.
+    if (n > 1 && std::find(lp.team.begin(), lp.team.end(), 0) == lp.team.end()) {
+        lp.classes.assign(1, all);
+        lp.team.assign(1, 1);
+        lp.tail.assign(1, 0u);
     }
 }
 
@@ -518,8 +541,10 @@ ce_status launch_classes(ce_engine* e, const LaunchPlan& lp, cek::KernelArgs a, 
     const size_t n = lp.classes.size();
     a.order = bk.order;
     a.chunk_k = e->chunk_k;
-    // Teams first: they leave room for the lanes' blocks, of which more start
-    // as the teams' ones end.
+    // Teams first, on as many blocks as fit: the lanes' blocks start as theirs
+    // end (ms on all blocks / half / a third of them: 150,000 bodies of the
+    // effects spec in the calm world x 5 s 174 / 225 / 262, 40,000 refine
+    // bodies x 3 s 55 / 61 / 70, 60,000 effects bodies x 5 s 66 / 63 / 70).
     for (int lanes = 0; lanes < 2; lanes++) {
         for (size_t c = 0; c < n; c++) {
             if ((lp.team[c] != 0) != (lanes == 0)) continue;
@@ -534,8 +559,7 @@ ce_status launch_classes(ce_engine* e, const LaunchPlan& lp, cek::KernelArgs a, 
             a.mm = k.mm;
             const cudaStream_t on = c == 0 ? st : side;
             if (lanes == 0) {
-                const cek::TeamSpec ts{flags, rate, cek::team_blocks(a.rows, a.count), (unsigned)e->sms, on,
-                                       n > 1 ? 2u : 1u};
+                const cek::TeamSpec ts{flags, rate, cek::team_blocks(a.rows, a.count), (unsigned)e->sms, on};
                 CE_TRY(cek::launch_team(ts, a, p), "advance launch");
                 continue;
             }
@@ -919,7 +943,9 @@ double device_load(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_
     return team_load(e, (double)count * team_cost(max_nodes, max_muscles), 0u, max_nodes, max_muscles);
 }
 unsigned device_tail(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_t max_muscles) {
-    return tail_most(e, count, device_load(e, count, max_nodes, max_muscles), 0.0, max_nodes, max_muscles);
+    const unsigned most =
+        tail_fit(e, count, device_load(e, count, max_nodes, max_muscles), 0.0, max_nodes, max_muscles);
+    return count > most ? most : 0u;  // a launch that is no larger starts on teams
 }
 }  // namespace
 

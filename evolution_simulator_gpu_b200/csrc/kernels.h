@@ -171,7 +171,6 @@ struct TeamSpec {
     int rate;
     unsigned blocks, sms;
     cudaStream_t stream;
-    unsigned share = 1u;  // leave the rest of the GPU to another launch: 1 / share of the blocks that fit
 };
 unsigned team_blocks(unsigned rows, size_t count);
 // Shared memory of a block for bodies of `first_n` to `rows` nodes.

@@ -36,7 +36,6 @@ cudaError_t team_one(const W& w, const TeamSpec& s, const KernelArgs& a, const c
     const cudaError_t e = team_occupancy_one<W, RECORD, RATE, CKPT>(warp_bytes, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    if (s.share > 1u && per_sm > 1) per_sm = (per_sm + (int)s.share - 1) / (int)s.share;
     const unsigned grid = s.blocks < (unsigned)per_sm * s.sms ? s.blocks : (unsigned)per_sm * s.sms;
     team_kernel<W, RECORD, RATE, CKPT>
         <<<grid > 0u ? grid : 1u, kTeamBlock, (size_t)warp_bytes * (kTeamBlock / 32u), s.stream>>>(a, p, w, warp_bytes);

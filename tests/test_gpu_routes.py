@@ -99,3 +99,18 @@ def test_a_backward_run_holds_tapes_for_its_teams_only(engine):
     with engine.forward(wave, w) as tape:
         tape.backward()
         assert free - torch.cuda.mem_get_info()[0] < 0.6e9
+
+
+@pytest.mark.parametrize("max_nodes,count", [(24, 40_000), (16, 60_000)])
+def test_two_classes(engine, lanes, max_nodes, count):
+    """Bodies of 3 to `max_nodes` nodes, of which the large ones alone would
+    pay for teams: beside the small ones' lanes they took 1.2 to 1.5 times as
+    long as both on lanes."""
+    w = ce.make_world(duration=0.5)
+    spec = ce.GenSpecPy(seed=5, min_nodes=3, max_nodes=max_nodes, muscle_rule=0, max_extra=3, joint_lo_deg=30.0,
+                        joint_hi_deg=150.0)
+    wave = ce.pack(ce.generate(spec, count), w)
+    a, b = engine.run(wave, w)[0], lanes.run(wave, w)[0]
+    assert (bits(a) == bits(b)).all()
+    mine, theirs = (min(e.run(wave, w)[1] for _ in range(4)) for e in (engine, lanes))
+    assert mine < 1.1 * theirs
