@@ -51,6 +51,11 @@ def class_kernels(count):
     return 2 if count >= TWO_KERNELS else int(count > 0)
 
 
+def device_kernels(count):
+    # On the device entry a kernel of its own sets the tail's length between the two.
+    return 3 if count >= TWO_KERNELS else int(count > 0)
+
+
 WORKLOAD_TEXT = ("3,000,000 seeded synthetic creatures (seed 1), 3-10 nodes, 2-24 muscles, calm flat world, "
                  "20 s trials at 60 steps/s x 16 substeps, FP32")
 
@@ -476,7 +481,7 @@ def run_engine(args):
             "parity": {"results_sha256": results_digest(res),
                        "compare_with": "the reference arm's reference_gpu.results_sha256: the reference kernel's "
                                        "results for the same generation in the same packed order"},
-            "gpu_launches": (BUCKET_KERNELS + class_kernels(len(wave))) * args.steps, "gpu_launches_e2e": e2e_launches,
+            "gpu_launches": (BUCKET_KERNELS + device_kernels(len(wave))) * args.steps, "gpu_launches_e2e": e2e_launches,
             "roofline": roofline, "cpu_baseline": cpu, "clocks": clk, "adjoint": adjoint, "effects": effects,
             "f3": f3,
         }

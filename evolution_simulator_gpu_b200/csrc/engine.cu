@@ -229,13 +229,10 @@ double lane_chain(unsigned nodes, unsigned muscles) {
     const double cached = 24u * nodes + 8u * muscles < 240u ? 250.0 * nodes : 0.0;
     return std::max(1200.0 * nodes + 280.0 * muscles - 1300.0 - cached, 500.0 * nodes);
 }
-// A creature's share of a substep of all schedulers on teams: its team's
-// lanes take turns at the muscles.
+// A creature's share of a substep of all schedulers on teams.
 double team_cost(unsigned nodes, unsigned muscles) {
     const unsigned lanes = nodes <= 8u ? 8u : nodes <= 16u ? 16u : 32u;
-    const double base = lanes == 8u ? 0.13 + 0.05 * nodes : (lanes == 16u ? 0.5 : 1.34) + 0.0385 * nodes;
-    const unsigned turns = std::max(1u, (muscles + lanes - 1u) / lanes);
-    return base + 0.0072 * lanes * turns;
+    return cek::team_cost(nodes, std::max(1u, (muscles + lanes - 1u) / lanes));
 }
 // Where the creatures' shared memory leaves room for fewer blocks an SM than
 // 8, latency shows (96 muscles on 8 lanes: 3 blocks, 1.44 ns instead of 0.9).
@@ -517,12 +514,17 @@ ce_status plan_launch(ce_engine* e, const ce_wave_pack* pack, uint32_t flags, in
     return CE_OK;
 }
 
-// A lane launch, and after it a team launch for the creatures it hands over.
+// A lane launch, and after it a team launch for the creatures it hands over:
+// the last `most`, or with a `budget` fewer (launch_tail_start).
 ce_status launch_lanes(ce_engine* e, const cek::LaunchSpec& ls, cek::KernelArgs a, const ce_params& p, void* tail,
-                       unsigned most) {
+                       unsigned most, double budget = 0.0) {
     if (most) {
         a.tail = cek::tail_layout(tail, most);
-        CE_TRY(cudaMemsetAsync(a.tail.counters, 0, cek::kTailCounters * 4u, ls.stream), "cudaMemsetAsync");
+        if (budget > 0.0) {
+            CE_TRY(cek::launch_tail_start(a.tail, a.bounds, a.work, a.count, budget, ls.stream), "tail launch");
+        } else {
+            CE_TRY(cudaMemsetAsync(a.tail.counters, 0, cek::kTailCounters * 4u, ls.stream), "cudaMemsetAsync");
+        }
     }
     CE_TRY(cek::launch_advance(ls, a, p), "advance launch");
     if (most) {
@@ -938,14 +940,17 @@ size_t slots_part(ce_engine* e, uint32_t world_flags, uint32_t rate, uint32_t ma
     if (e->opened_ctas) take(e->opened_ctas);
     return (scratch_bytes(grid, max_nodes, max_muscles, false) + 255u) & ~(size_t)255u;
 }
-// Only the largest body is known here: every creature is taken for one.
+// Only the largest body is known here: for the choice of teams every creature
+// is taken for one. The tail's is made on the device, from the queues; its
+// area holds what it can come to.
 double device_load(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_t max_muscles) {
     return team_load(e, (double)count * team_cost(max_nodes, max_muscles), 0u, max_nodes, max_muscles);
 }
 unsigned device_tail(const ce_engine* e, size_t count, uint32_t max_nodes, uint32_t max_muscles) {
-    const unsigned most =
-        tail_fit(e, count, device_load(e, count, max_nodes, max_muscles), 0.0, max_nodes, max_muscles);
-    return count > most ? most : 0u;  // a launch that is no larger starts on teams
+    if (!e->teams || e->tuning || device_load(e, count, max_nodes, max_muscles) <= lane_chain(max_nodes, max_muscles)) {
+        return 0u;
+    }
+    return (unsigned)std::min<size_t>(count, kTeamMost);
 }
 }  // namespace
 
@@ -1013,7 +1018,8 @@ ce_status advance_device(ce_engine* e, const uint32_t* records, const float* mus
     const cek::LaunchSpec ls{max_nodes, max_muscles, world_flags, false, (int)rate, grid, cek::kBlock, st};
     char* const tail = static_cast<char*>(scratch) + slots_part(e, world_flags, rate, max_nodes, max_muscles) +
                        cek::bucket_bytes(params->count);
-    return launch_lanes(e, ls, a, *params, tail, device_tail(e, a.count, max_nodes, max_muscles));
+    const double budget = 0.75 * lane_chain(max_nodes, max_muscles) / team_load(e, 1.0, 0u, max_nodes, max_muscles);
+    return launch_lanes(e, ls, a, *params, tail, device_tail(e, a.count, max_nodes, max_muscles), budget);
 }
 }  // namespace
 

@@ -58,6 +58,18 @@ constexpr unsigned kTailDone = 0, kTailStates = 1, kTailWritten = 2, kTailClaime
 __host__ __device__ inline unsigned tail_floats(unsigned rows, unsigned mm) { return 4u * rows + 2u * mm + 34u; }
 size_t tail_bytes(unsigned rows, unsigned mm, unsigned most);
 Tail tail_layout(void* area, unsigned most);
+// A creature's share of a substep of all schedulers on teams, ns on 148 SMs:
+// its team's lanes take `turns` at the muscles (engine.cu has the measure).
+__host__ __device__ inline double team_cost(unsigned nodes, double turns) {
+    const unsigned lanes = nodes <= 8u ? 8u : nodes <= 16u ? 16u : 32u;
+    const double base = lanes == 8u ? 0.13 + 0.05 * nodes : (lanes == 16u ? 0.5 : 1.34) + 0.0385 * nodes;
+    return base + 0.0072 * lanes * turns;
+}
+// Starts a tail's counters for a launch whose bodies only the device knows, by
+// its queues of every node count (`bounds`, `work`): it hands over once no more
+// are left than cost `budget` ns a substep on teams, and at most tail.most.
+cudaError_t launch_tail_start(const Tail& tail, const uint32_t* bounds, const unsigned long long* work,
+                              uint32_t count, double budget, cudaStream_t stream);
 
 struct KernelArgs {
     const uint32_t* records;

@@ -595,8 +595,8 @@ ce_status ce_graph_close(ce_graph* graph);
  * GPU time. ce_gene_gradients maps the record gradients to genes. The tape
  * holds device memory until ce_tape_free: beside the batch, its gradients and
  * 16 (rows + muscle slots / 4) bytes a checkpoint, a segment's states: on
- * teams of lanes 1.2 MB a warp (4, 2 or 1 bodies of up to 8, 16 or 32 nodes)
- * and at most 1.5 GB, on lanes 256 states a lane and at most 3 GB. */
+ * teams of lanes 1.2 to 1.6 MB a warp (4, 2 or 1 bodies of up to 8, 16 or 32
+ * nodes) and at most 1.9 GB, on lanes 256 states a lane and at most 3 GB. */
 typedef struct ce_tape ce_tape;
 ce_status ce_forward(ce_engine* engine, const ce_wave_pack* pack, const ce_world* world,
                      uint32_t checkpoint_every, ce_tape** tape);
